@@ -7,10 +7,20 @@
 // the singular system consistent; the gauge is fixed by mean(p) = 0.
 //
 // Outer loop (FP64): defect correction.  r = b - A p in FP64; stop when
-// ||r|| <= tol ||b||; otherwise one multigrid V-cycle approximates A e = r
-// in the inner precision and p += e in FP64.  The inner solve:
+// ||r|| <= tol ||b||; otherwise an inner solve of A e = r and p += e in FP64.
+// The inner solve, on grids of at least MG_DIRECT_CELLS cells: the direct one
+// of spectral.cu, FP64 in both modes, whose residual is at rounding (1e-15 to
+// 4e-11 of b from 24^3 to a 900-cell side), so one correction meets any
+// tolerance above that.  A solve of the 200^3 dam break takes 0.62 ms on a
+// B200 where 8 to 9 V-cycles took 2.7 (MIXED) and 4.6 ms (FP64); 100 x 80 x
+// 126 (10 V-cycles) 0.16 where it was 3.1 ms; 24^3 0.09 where it was 0.6-0.8.
+// Smaller grids keep one multigrid V-cycle per correction: programs there
+// read the cycle count and meet its cap (solver_stats, max_outer), which a
+// direct solve would always leave at 1.  Its vectors:
 //   MIXED: every multigrid vector stored in BF16, arithmetic in FP32;
 //   FP64:  the same cycle with FP64 storage and arithmetic (the yardstick).
+// VOF_MG_PAIRS (0 or 1: row or paired kernels) in the environment keeps the
+// V-cycle at any size, as a check of one solver against the other.
 // V-cycle: Chebyshev-accelerated Jacobi (the Jacobi update of the reference's
 // sweep inside the Chebyshev three-term recurrence) as the smoother, degree 3
 // before and after on levels wider than 25 cells (eigenvalues of D^-1 A in
@@ -41,6 +51,7 @@
 #include <vector>
 
 #include "mg_solve.h"
+#include "pdl.cuh"
 
 namespace vof {
 
@@ -63,34 +74,6 @@ struct St<double> {
 
 constexpr int MG_THREADS = MG_BX * MG_BY;
 constexpr int TAIL_THREADS = 1024;
-
-// Programmatic dependent launch.  Every kernel of the solve is launched with
-// cudaLaunchAttributeProgrammaticStreamSerialization (pdl_launch) and begins
-// with pdl_enter(): it waits for the grid before it to complete (and its
-// writes to be visible) before its first global memory access, then lets the
-// next grid launch.  The launch and prologue of a kernel so overlap the end of
-// the one before, which removes most of the gap between the short kernels of
-// the coarse levels.  Launched without the attribute, the wait returns at once.
-__device__ __forceinline__ void pdl_enter() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-
-template <typename... KArgs, typename... Args>
-static cudaError_t pdl_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
-                              Args&&... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
-}
 
 __host__ __device__ __forceinline__ int nb_count(int x, int n) { return (x > 0) + (x < n - 1); }
 
@@ -1127,6 +1110,18 @@ static bool dense_inverse(const MgLevel& L, std::vector<double>& inv) {
     return true;
 }
 
+// Direct solve: planes per thread and threads per block of the passes over the fields.
+constexpr int DK = 2, D_THREADS = 256;
+// Planes per block: about four waves of blocks (four of k_dresid's fit an SM), at least 4 planes.
+static int direct_chunk(const Geom& g) {
+    const int bx = (g.nx * g.ny + D_THREADS - 1) / D_THREADS;
+    const int z = (4 * 4 * 148 + bx - 1) / bx, kc = (g.nz + z - 1) / z;
+    return kc < 4 ? 4 : kc;
+}
+static dim3 direct_grid(const Geom& g, int kc) {
+    return dim3((g.nx * g.ny + D_THREADS - 1) / D_THREADS, (g.nz + kc - 1) / kc);
+}
+
 cudaError_t mg_create(const Geom& g, int mode, MgSolver* m, cudaStream_t s, size_t* bytes, int* alloc_no,
                       int fail_at) {
     *m = MgSolver{};
@@ -1134,19 +1129,21 @@ cudaError_t mg_create(const Geom& g, int mode, MgSolver* m, cudaStream_t s, size
     m->pairs = 1;
     if (const char* v = getenv("VOF_MG_PAIRS")) m->pairs = atoi(v) != 0;
     m->nlev = mg_plan(g, m->lv, MG_MAX_LEVELS);
+    m->direct = m->lv[0].ncell >= MG_DIRECT_CELLS && !getenv("VOF_MG_PAIRS");
+    if (m->direct) m->nlev = 1;
     cudaError_t e;
-    const size_t vb = mode == MG_MIXED ? sizeof(__nv_bfloat16) : sizeof(double);
+    const size_t vb = m->direct ? sizeof(double) : mode == MG_MIXED ? sizeof(__nv_bfloat16) : sizeof(double);
     const size_t cb = mode == MG_MIXED ? sizeof(float) : sizeof(double);
     const MgLevel& Lc = m->lv[m->nlev - 1];
     // The tail: the deepest run of levels (at most MG_TAIL_CELLS cells each)
     // whose vectors and dense coarse inverse fit in MG_TAIL_SMEM bytes.
-    const bool dense_ok = Lc.ncell <= MG_DENSE_MAX;
+    const bool dense_ok = !m->direct && Lc.ncell <= MG_DENSE_MAX;
     const size_t inv_bytes = dense_ok ? (size_t)Lc.ncell * Lc.ncell * cb : 0;
     m->tail = m->nlev;
     m->tail_smem = 0;
     {
         size_t acc = inv_bytes;
-        for (int l = m->nlev - 1; l >= 0; --l) {
+        for (int l = m->nlev - 1; l >= 0 && !m->direct; --l) {
             const size_t lb = 3 * (size_t)tail_vec_bytes(m->lv[l].ncell, (int)vb);
             if (m->lv[l].ncell > MG_TAIL_CELLS || acc + lb > MG_TAIL_SMEM) break;
             acc += lb;
@@ -1179,18 +1176,24 @@ cudaError_t mg_create(const Geom& g, int mode, MgSolver* m, cudaStream_t s, size
     for (int l = 0; l < m->nlev; ++l) {
         MgLevel& L = m->lv[l];
         const size_t nb = (size_t)L.ncell * vb;
-        if ((e = alloc(&L.e0, nb)) != cudaSuccess || (e = alloc(&L.e1, nb)) != cudaSuccess ||
-            (e = alloc(&L.b, nb)) != cudaSuccess)
-            return e;
+        if ((e = alloc(&L.b, nb)) != cudaSuccess) return e;
+        if (!m->direct && ((e = alloc(&L.e0, nb)) != cudaSuccess || (e = alloc(&L.e1, nb)) != cudaSuccess)) return e;
         const int blk = L.gx * L.gy * L.gz;
         maxblk = blk > maxblk ? blk : maxblk;
     }
     m->nblk = m->lv[0].gx * m->lv[0].gy * m->lv[0].gz;
+    if (m->direct) {
+        const dim3 dg = direct_grid(g, direct_chunk(g));
+        maxblk = (3 * (int)(dg.x * dg.y) + 1) / 2;
+        if ((e = sp_create(g, &m->sp, s, alloc)) != cudaSuccess ||
+            (e = alloc((void**)&m->d_ticket, sizeof(unsigned))) != cudaSuccess)
+            return e;
+    }
     if ((e = alloc((void**)&m->d_partial, sizeof(double) * 2 * maxblk)) != cudaSuccess ||
         (e = alloc((void**)&m->d_result, sizeof(double) * 8)) != cudaSuccess ||
         (e = alloc((void**)&m->d_lv, sizeof(MgLevel) * m->nlev)) != cudaSuccess)
         return e;
-    if ((e = cudaHostAlloc((void**)&m->h_result, sizeof(double) * 2, cudaHostAllocMapped)) != cudaSuccess) {
+    if ((e = cudaHostAlloc((void**)&m->h_result, sizeof(double) * 4, cudaHostAllocMapped)) != cudaSuccess) {
         m->h_result = nullptr;
         return e;
     }
@@ -1224,6 +1227,9 @@ void mg_destroy(MgSolver* m) {
     if (m->d_result) cudaFree(m->d_result);
     if (m->h_result) cudaFreeHost(m->h_result);
     if (m->iter_graph) cudaGraphExecDestroy(m->iter_graph);
+    if (m->first_graph) cudaGraphExecDestroy(m->first_graph);
+    if (m->d_ticket) cudaFree(m->d_ticket);
+    sp_destroy(&m->sp);
     *m = MgSolver{};
 }
 
@@ -1368,34 +1374,28 @@ static cudaError_t outer_iteration(const Geom& g, MgSolver& m, const R* rhs, dou
     return cudaGetLastError();
 }
 
-template <typename S, typename R>
-static cudaError_t capture_iteration(const Geom& g, MgSolver& m, const R* rhs, double* p64, float* p32,
-                                     cudaStream_t cap) {
-    if (m.iter_graph) {
-        cudaGraphExecDestroy(m.iter_graph);
-        m.iter_graph = nullptr;
+// The kernels that `enqueue(cap, launches)` puts on the capture stream, as an executable graph.
+template <typename Enqueue>
+static cudaError_t capture(cudaStream_t cap, cudaGraphExec_t* exec, int* kernels, Enqueue&& enqueue) {
+    if (*exec) {
+        cudaGraphExecDestroy(*exec);
+        *exec = nullptr;
     }
     cudaError_t e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return e;
     int launches = 0;
-    const cudaError_t e1 = outer_iteration<S, R>(g, m, rhs, p64, cap, launches);
+    const cudaError_t e1 = enqueue(cap, launches);
     cudaGraph_t graph = nullptr;
     e = cudaStreamEndCapture(cap, &graph);
     if (e1 != cudaSuccess || e != cudaSuccess) {
         if (graph) cudaGraphDestroy(graph);
         return e1 != cudaSuccess ? e1 : e;
     }
-    e = cudaGraphInstantiate(&m.iter_graph, graph, 0);
+    e = cudaGraphInstantiate(exec, graph, 0);
     cudaGraphDestroy(graph);
-    if (e != cudaSuccess) {
-        m.iter_graph = nullptr;
-        return e;
-    }
-    m.graph_key[0] = rhs;
-    m.graph_key[1] = p64;
-    m.graph_key[2] = p32;
-    m.graph_launches = launches;
-    return cudaSuccess;
+    if (e != cudaSuccess) *exec = nullptr;
+    *kernels = launches;
+    return e;
 }
 
 template <typename S, typename R>
@@ -1406,8 +1406,15 @@ static cudaError_t solve_impl(const Geom& g, MgSolver& m, const R* rhs, double* 
     double* part = m.d_partial;
     double* res = m.d_result;
     cudaError_t e;
-    if (!m.iter_graph || m.graph_key[0] != rhs || m.graph_key[1] != p64 || m.graph_key[2] != p32)
-        if ((e = capture_iteration<S, R>(g, m, rhs, p64, p32, cap)) != cudaSuccess) return e;
+    if (!m.iter_graph || m.graph_key[0] != rhs || m.graph_key[1] != p64 || m.graph_key[2] != p32) {
+        e = capture(cap, &m.iter_graph, &m.graph_launches, [&](cudaStream_t c, int& n) {
+            return outer_iteration<S, R>(g, m, rhs, p64, c, n);
+        });
+        if (e != cudaSuccess) return e;
+        m.graph_key[0] = rhs;
+        m.graph_key[1] = p64;
+        m.graph_key[2] = p32;
+    }
     int launches = 0;
     pdl_launch(k_sum_rhs<R>, grid, kBlock, 0, s, g, L0, rhs, part);
     pdl_launch(k_fold2, 1, MG_THREADS, 0, s, part, m.nblk, res + 2, nullptr);
@@ -1440,8 +1447,243 @@ static cudaError_t solve_impl(const Geom& g, MgSolver& m, const R* rhs, double* 
     return rel <= tol ? cudaSuccess : cudaErrorNotReady;
 }
 
+// ---- the direct solve (spectral.cu) ---------------------------------------------
+// FP64 passes over the padded fields around sp_correct.  Threads are numbered
+// flat over a plane's cells (no idle lanes at row ends) and march a chunk of
+// planes.
+// Each pass with a sum folds its blocks' partials in its last block, in a
+// fixed order.
+// Sums of a block's threads into partial[3 b ..]; the last block of the grid
+// to arrive folds them into out[0 .. 2] (every launch leaves ticket at 0).
+__device__ __forceinline__ void fold3(double a, double b, double c, double* partial, unsigned* ticket, double* out,
+                                      double* host_out) {
+    __shared__ double sh[3][D_THREADS / 32];
+    __shared__ bool last;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned nblk = gridDim.x * gridDim.y, blk = blockIdx.y * gridDim.x + blockIdx.x;
+    auto sum = [&]() {
+        for (int o = 16; o > 0; o >>= 1) {
+            a += __shfl_down_sync(0xffffffffu, a, o);
+            b += __shfl_down_sync(0xffffffffu, b, o);
+            c += __shfl_down_sync(0xffffffffu, c, o);
+        }
+        if (lane == 0) {
+            sh[0][warp] = a;
+            sh[1][warp] = b;
+            sh[2][warp] = c;
+        }
+        __syncthreads();
+        a = b = c = 0.0;
+        if (threadIdx.x == 0)
+            for (int w = 0; w < D_THREADS / 32; ++w) {
+                a += sh[0][w];
+                b += sh[1][w];
+                c += sh[2][w];
+            }
+    };
+    sum();
+    if (threadIdx.x == 0) {
+        partial[3 * blk] = a;
+        partial[3 * blk + 1] = b;
+        partial[3 * blk + 2] = c;
+        __threadfence();
+        last = atomicInc(ticket, nblk - 1) == nblk - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    a = b = c = 0.0;
+#pragma unroll 4
+    for (unsigned q = threadIdx.x; q < nblk; q += D_THREADS) {
+        a += __ldcg(partial + 3 * q);
+        b += __ldcg(partial + 3 * q + 1);
+        c += __ldcg(partial + 3 * q + 2);
+    }
+    sum();
+    if (threadIdx.x == 0) {
+        out[0] = a;
+        out[1] = b;
+        out[2] = c;
+        if (host_out) {
+            host_out[0] = a;
+            host_out[1] = b;
+            __threadfence_system();
+        }
+    }
+}
+
+struct DCell {
+    int i, j, k0, k1, id;
+    bool live;
+    __device__ DCell(const Geom& g, int kchunk) {
+        const int q = blockIdx.x * D_THREADS + threadIdx.x;
+        live = q < g.nx * g.ny;
+        i = live ? q % g.nx : 0;
+        j = live ? q / g.nx : 0;
+        k0 = 1 + blockIdx.y * kchunk;
+        k1 = live ? min(g.nz, k0 + kchunk - 1) : 0;
+        id = gidx(g, i + 1, j + 1, k0);
+    }
+};
+
+template <typename R>
+__global__ void __launch_bounds__(D_THREADS) k_dsum(Geom g, int kchunk, const R* __restrict__ rhs, double* partial,
+                                                    unsigned* ticket, double* out) {
+    pdl_enter();
+    const DCell t(g, kchunk);
+    double a = 0.0;
+    int id = t.id;
+#pragma unroll 8
+    for (int k = t.k0; k <= t.k1; ++k, id += g.plane) a += (double)rhs[id];
+    fold3(a, 0.0, 0.0, partial, ticket, out, nullptr);
+}
+
+// r = (rhs - mean) - A p (STORE: into r0, compact); the sums of r^2, of
+// (rhs - mean)^2 and of p.  A thread marches a chunk of planes DK at a time,
+// the operands of a step loaded together.
+template <typename R, bool STORE>
+__global__ void __launch_bounds__(D_THREADS, 4) k_dresid(Geom g, int kchunk, double ax, double ay, double az,
+                                                         const R* __restrict__ rhs, const double* __restrict__ sums,
+                                                         const double* __restrict__ p, double* __restrict__ r0,
+                                                         double* partial, unsigned* ticket, double* out,
+                                                         double* host_out) {
+    pdl_enter();
+    const DCell t(g, kchunk);
+    double rr = 0.0, bb = 0.0, pp = 0.0;
+    const double mean = sums[0] / ((double)g.nx * g.ny * g.nz);
+    // a wall's neighbour is the cell itself (its difference is 0)
+    const int ow = t.i > 0 ? -1 : 0, oe = t.i < g.nx - 1 ? 1 : 0;
+    const int os = t.j > 0 ? -g.px : 0, on = t.j < g.ny - 1 ? g.px : 0;
+    int id = t.id, c0 = ((t.k0 - 1) * g.ny + t.j) * g.nx + t.i;
+    double pm = 0.0, pc = 0.0;
+    if (t.k1 > 0) {
+        pc = p[id];
+        pm = t.k0 > 1 ? p[id - g.plane] : pc;
+    }
+    for (int k = t.k0; k <= t.k1; k += DK, id += DK * g.plane, c0 += DK * g.nx * g.ny) {
+        double c[DK + 1], w[DK], e[DK], s[DK], n[DK], b[DK];
+        c[0] = pc;
+#pragma unroll
+        for (int q = 0; q < DK; ++q) {
+            const int at = id + (k + q <= t.k1 ? q : 0) * g.plane;
+            c[q + 1] = p[k + q < g.nz ? at + g.plane : at];
+            w[q] = p[at + ow];
+            e[q] = p[at + oe];
+            s[q] = p[at + os];
+            n[q] = p[at + on];
+            b[q] = (double)rhs[at];
+        }
+#pragma unroll
+        for (int q = 0; q < DK; ++q) {
+            if (k + q > t.k1) break;
+            const double x = c[q];
+            double v = ax * (w[q] - x);
+            v += ax * (e[q] - x);
+            v += ay * (s[q] - x);
+            v += ay * (n[q] - x);
+            v += az * (pm - x);
+            v += az * (c[q + 1] - x);
+            const double f = b[q] - mean, r = f - v;
+            rr += r * r;
+            bb += f * f;
+            pp += x;
+            if (STORE) r0[c0 + q * g.nx * g.ny] = r;
+            pm = x;
+            pc = c[q + 1];
+        }
+    }
+    fold3(rr, bb, pp, partial, ticket, out, host_out);
+}
+
+// p -= mean(p) (gauge), p32 = float(p) on the interior.
+__global__ void __launch_bounds__(D_THREADS) k_dgauge(Geom g, int kchunk, const double* __restrict__ sum,
+                                                      double* __restrict__ p, float* __restrict__ p32) {
+    pdl_enter();
+    const DCell t(g, kchunk);
+    const double mean = sum[0] / ((double)g.nx * g.ny * g.nz);
+    int id = t.id;
+    for (int k = t.k0; k <= t.k1; k += 4, id += 4 * g.plane) {
+        double v[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) v[q] = k + q <= t.k1 ? p[id + q * g.plane] - mean : 0.0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            if (k + q > t.k1) break;
+            p[id + q * g.plane] = v[q];
+            if (p32) p32[id + q * g.plane] = (float)v[q];
+        }
+    }
+}
+
+// One captured graph: (first) the mean of rhs, the residual of the start
+// value; the correction, the new residual and the gauge.  The corrections'
+// kernels return at once where the start value meets the tolerance already,
+// so the host waits once per solve, not before it; a solve that needs more
+// (tolerances near rounding) launches the second graph, without the mean, again.
+template <typename R>
+static cudaError_t direct_pass(const Geom& g, MgSolver& m, const R* rhs, double* p64, float* p32, double tol, bool first,
+                               cudaStream_t s, int& launches) {
+    const MgLevel& L = m.lv[0];
+    const int kc = direct_chunk(g);
+    const dim3 grid = direct_grid(g, kc);
+    double* r = static_cast<double*>(L.b);
+    double* res = m.d_result;  // [0..2] norms and sum of p, [3..5] sum of rhs
+    if (first) {
+        pdl_launch(k_dsum<R>, grid, D_THREADS, 0, s, g, kc, rhs, m.d_partial, m.d_ticket, res + 3);
+        ++launches;
+    }
+    pdl_launch(k_dresid<R, true>, grid, D_THREADS, 0, s, g, kc, L.ax, L.ay, L.az, rhs, (const double*)(res + 3),
+               (const double*)p64, r, m.d_partial, m.d_ticket, res, m.h_result_dev);
+    cudaError_t e = sp_correct(g, m.sp, r, p64, SpStop{res, tol}, s, launches);
+    if (e != cudaSuccess) return e;
+    pdl_launch(k_dresid<R, false>, grid, D_THREADS, 0, s, g, kc, L.ax, L.ay, L.az, rhs, (const double*)(res + 3),
+               (const double*)p64, (double*)nullptr, m.d_partial, m.d_ticket, res, m.h_result_dev + 2);
+    pdl_launch(k_dgauge, grid, D_THREADS, 0, s, g, kc, (const double*)(res + 2), p64, p32);
+    launches += 3;
+    return cudaGetLastError();
+}
+
+template <typename R>
+static cudaError_t direct_solve(const Geom& g, MgSolver& m, const R* rhs, double* p64, float* p32, double tol,
+                                int max_outer, MgStats* st, cudaStream_t s, cudaStream_t cap) {
+    cudaError_t e;
+    if (!m.iter_graph || m.graph_key[0] != rhs || m.graph_key[1] != p64 || m.graph_key[2] != p32 || m.graph_tol != tol) {
+        e = capture(cap, &m.first_graph, &m.first_launches,
+                    [&](cudaStream_t c, int& n) { return direct_pass(g, m, rhs, p64, p32, tol, true, c, n); });
+        if (e != cudaSuccess) return e;
+        e = capture(cap, &m.iter_graph, &m.graph_launches,
+                    [&](cudaStream_t c, int& n) { return direct_pass(g, m, rhs, p64, p32, tol, false, c, n); });
+        if (e != cudaSuccess) return e;
+        m.graph_key[0] = rhs;
+        m.graph_key[1] = p64;
+        m.graph_key[2] = p32;
+        m.graph_tol = tol;
+    }
+    const auto rel = [&](int q) { return m.h_result[q + 1] > 0 ? sqrt(m.h_result[q] / m.h_result[q + 1]) : 0.0; };
+    if ((e = cudaGraphLaunch(m.first_graph, s)) != cudaSuccess || (e = cudaStreamSynchronize(s)) != cudaSuccess)
+        return e;
+    const double r0 = rel(0);
+    double now = rel(2);
+    int it = r0 <= tol ? 0 : 1, launches = m.first_launches;
+    while (it > 0 && !(now <= tol) && it < max_outer) {
+        if ((e = cudaGraphLaunch(m.iter_graph, s)) != cudaSuccess || (e = cudaStreamSynchronize(s)) != cudaSuccess)
+            return e;
+        now = rel(2);
+        launches += m.graph_launches;
+        ++it;
+    }
+    if (st) {
+        st->outer = it;
+        st->rel_initial = r0;
+        st->rel_final = now;
+        st->launches = launches;
+    }
+    return now <= tol ? cudaSuccess : cudaErrorNotReady;
+}
+
 cudaError_t mg_solve(const Geom& g, MgSolver& m, const float* rhs, double* p64, float* p32, double tol,
                      int max_outer, MgStats* st, cudaStream_t s, cudaStream_t cap) {
+    if (m.direct) return direct_solve<float>(g, m, rhs, p64, p32, tol, max_outer, st, s, cap);
     if (m.mode == MG_MIXED)
         return solve_impl<__nv_bfloat16, float>(g, m, rhs, p64, p32, tol, max_outer, st, s, cap);
     return solve_impl<double, float>(g, m, rhs, p64, p32, tol, max_outer, st, s, cap);
@@ -1449,6 +1691,7 @@ cudaError_t mg_solve(const Geom& g, MgSolver& m, const float* rhs, double* p64, 
 
 cudaError_t mg_solve64(const Geom& g, MgSolver& m, const double* rhs, double* p64, double tol, int max_outer,
                        MgStats* st, cudaStream_t s, cudaStream_t cap) {
+    if (m.direct) return direct_solve<double>(g, m, rhs, p64, nullptr, tol, max_outer, st, s, cap);
     if (m.mode == MG_MIXED)
         return solve_impl<__nv_bfloat16, double>(g, m, rhs, p64, nullptr, tol, max_outer, st, s, cap);
     return solve_impl<double, double>(g, m, rhs, p64, nullptr, tol, max_outer, st, s, cap);

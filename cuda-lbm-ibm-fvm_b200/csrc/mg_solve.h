@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 #include <stddef.h>
 
+#include "spectral.h"
 #include "vof_device.cuh"
 
 namespace vof {
@@ -17,6 +18,8 @@ constexpr double MG_RATIO_FINE = 6.0;   // eigenvalue ratio they damp (the 2x-co
 constexpr int MG_NU_COARSE = 8;         // pre/post degree on the small levels
 constexpr double MG_RATIO_COARSE = 30.0;  // wider: these levels may coarsen by 3, 5 or 7
 constexpr int MG_MAX_NU = 8;
+// Grids of at least this many cells are solved directly (spectral.cu).
+constexpr int MG_DIRECT_CELLS = 8192;
 constexpr int MG_COARSE_SWEEPS = 100;   // sweeps on a coarsest level too large for the dense solve
 constexpr int MG_MAX_LEVELS = 16;
 constexpr int MG_TAIL_CELLS = 4096;     // largest level that may run inside the one-block kernel
@@ -56,6 +59,8 @@ struct MgSolver {
     // levels of even width and for 2x2x2 coarsening; 0: the row kernels
     // (VOF_MG_PAIRS=0)
     int pairs;
+    int direct;      // the inner solve is the direct one, sp (one level, no cycle)
+    SpSolver sp;
     int nlev;
     int tail;        // first level handled by the one-block kernel (nlev: none)
     int dense;       // the coarsest level is solved with the stored inverse
@@ -66,12 +71,18 @@ struct MgSolver {
     double* d_partial;  // reduction partials, 2 per block of the largest tiling
     int nblk;           // blocks of the fine tiling
     double* d_result;   // [0..1] residual sums, [2..3] sum of rhs, [4..5] sum of p, [6..7] coarse mean
-    double* h_result;   // mapped pinned host copy of the residual sums (2 doubles)
+    double* h_result;   // mapped pinned host copy of the residual sums (2 doubles; direct solve: before and after)
     double* h_result_dev;  // its device alias
     // One outer iteration (V-cycle, p += e, new residual) captured once as a graph.
     cudaGraphExec_t iter_graph;
     const void* graph_key[3];  // rhs, p64, p32 the graph was captured with
     int graph_launches;        // kernels in it
+    // direct solve: the first iteration (with the mean of rhs) captured too,
+    // for this tolerance; ticket of the passes' last-block folds
+    cudaGraphExec_t first_graph;
+    int first_launches;
+    double graph_tol;
+    unsigned* d_ticket;
 };
 
 struct MgStats {

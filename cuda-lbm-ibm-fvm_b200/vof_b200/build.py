@@ -36,12 +36,13 @@ SOURCES = {
     "adjoint.cu": ["-fmad=false", "-DVOF_FMAD_FALSE"],
     "tma_host.cu": [],
     "mg_solve.cu": [],
+    "spectral.cu": [],
     "reduce.cu": [],
     "capi.cu": [],
     "noalloc.cu": [],
     "apply_bc.cu": [],
 }
-HEADERS = ["vof_device.cuh", "tma.cuh", "plain_step.h", "fct_sweep.h", "fct_line.cuh", "jacobi_tb.h", "mg_solve.h",
+HEADERS = ["vof_device.cuh", "tma.cuh", "plain_step.h", "fct_sweep.h", "fct_line.cuh", "jacobi_tb.h", "mg_solve.h", "spectral.h", "pdl.cuh",
            "reduce.h", "adjoint.h", "apply_bc.h"]
 
 

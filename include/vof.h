@@ -45,8 +45,10 @@ extern "C" {
 
 /* ---- solver modes ------------------------------------------------------ */
 #define VOF_MODE_PLAIN  0   /* FP32, jacobi_iters Jacobi sweeps: the drop-in path */
-#define VOF_MODE_MIXED  1   /* FP64 defect correction over a BF16-stored/FP32 inner solve */
-#define VOF_MODE_FP64   2   /* same convergent projection, every field in FP64    */
+/* Both: FP64 defect correction.  Grids of at least 8192 cells: each correction
+   is a direct FP64 solve (cosine transforms).  Smaller grids: one V-cycle, */
+#define VOF_MODE_MIXED  1   /* ... BF16-stored / FP32 arithmetic */
+#define VOF_MODE_FP64   2   /* ... FP64 */
 
 /* ---- field identifiers (vof_upload / vof_download) --------------------- */
 #define VOF_FIELD_F      0  /* volume fraction (DeviceFields::F)      */
@@ -93,9 +95,8 @@ typedef struct vof_params {
     /* ---- additions (no counterpart in Params) ---- */
     int jacobi_iters;       /* plain mode: sweeps per step; voftrial1.cu:1371 hardcodes 10 */
     int mode;               /* VOF_MODE_*                                                   */
-    int inner_sweeps;       /* reserved (kept for the ABI layout): the multigrid inner solve of the
-                               mixed/fp64 modes uses fixed Chebyshev smoothing degrees (3 on levels
-                               wider than 25 cells, 8 below); vof_params_init sets 32, unused */
+    int inner_sweeps;       /* reserved (kept for the ABI layout): the inner solve of the
+                               mixed/fp64 modes takes no such count; vof_params_init sets 32, unused */
     int max_outer;          /* mixed/fp64 modes: cap on defect-correction iterations        */
     double tol;             /* mixed/fp64 modes: target ||b-Ap||/||b|| (default 1e-8)       */
     int surface_tension;    /* 1: add the continuum-surface-force acceleration sigma kappa
@@ -286,7 +287,7 @@ int vof_apply_bc_fields(const vof_params* p, float* u, float* v, float* w, float
 
 /*
  * Convergent modes (VOF_MODE_MIXED, VOF_MODE_FP64; no counterpart in the
- * reference): V-cycles done by the last pressure solve and its relative
+ * reference): corrections (inner solves) done by the last pressure solve and its relative
  * residual ||b - A p|| / ||b|| (FP64, b = rhs - mean) at entry and at exit.
  * VOF_E_STATE in VOF_MODE_PLAIN.
  */
