@@ -59,21 +59,19 @@ UNIT = "Mcell-updates/s"
 ALG_BYTES = {
     "predict": 28,   # read F,u,v,w; write u*,v*,w*
     "rhs": 20,       # read F,u*,v*,w*; write rhs
-    "jacobi": 12,    # read rhs,p; write p'
+    "jacobi": 12,    # a launch (two sweeps): read rhs,p; write p'
     "correct": 32,   # read u*,v*,w*,p,F; write u,v,w
     "sweep1": 12,    # read F, face velocity; write F
     "sweep2": 12,
     "sweep3": 12,
 }
 KERNEL_NAMES = {
-    "predict": "k_predict2", "rhs": "k_rhs4", "jacobi": "k_jacobi_peel", "correct": "k_correct4",
+    "predict": "k_predict2", "rhs": "k_rhs4", "jacobi": "k_jacobi_two", "correct": "k_correct4",
     "sweep1": "k_fct_x|k_fct_march", "sweep2": "k_fct_x|k_fct_march", "sweep3": "k_fct_x|k_fct_march",
 }
-# the Jacobi kernel the library runs at the bench size (VOF_JACOBI=peel|pairs|ring|bulk|col|pairs2|tb|tb1;
-# peel, one sweep per launch with two cells per thread, by default)
-KERNEL_NAMES["jacobi"] = {"col": "k_jacobi_col", "tb": "k_jacobi_tb", "tb1": "k_jacobi_tb", "pairs2": "k_jacobi_pairs2",
-                          "ring": "k_jacobi_ring", "bulk": "k_jacobi_bulk",
-                          "pairs": "k_jacobi_pairs"}.get(os.environ.get("VOF_JACOBI", ""), "k_jacobi_peel")
+# (VOF_JACOBI=peel: one sweep per launch; by default two, k_jacobi_two)
+if os.environ.get("VOF_JACOBI") == "peel":
+    KERNEL_NAMES["jacobi"] = "k_jacobi_peel"
 if os.environ.get("VOF_CORRECT") == "1":
     KERNEL_NAMES["correct"] = "k_correct"
 if os.environ.get("VOF_RHS") == "1":

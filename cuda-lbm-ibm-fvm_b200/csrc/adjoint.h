@@ -85,7 +85,7 @@ struct AdjEngine {
     bool recorded;
     // recompute buffers (FP32)
     PlainBuffers wb;
-    CUtensorMap maps[4];
+    J2Tables j2;              // of wb's p0, p1, p2, rhs
     int* status;
     float *Fin1, *Fin2, *Ftd, *A, *C, *rp, *rm;
     // adjoint fields (FP64)

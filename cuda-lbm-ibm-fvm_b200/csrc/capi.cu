@@ -12,7 +12,7 @@
 #include <new>
 
 #include "../../include/vof.h"
-#include "jacobi_tb.h"
+#include "jacobi_two.h"
 #include "adjoint.h"
 #include "apply_bc.h"
 #include "mg_solve.h"
@@ -42,7 +42,7 @@ struct vof_ctx {
     double* d_red_result;
     double* h_red_result;       // pinned, for vof_reduce
     int* d_status;              // device status word written by kernels (DEV_* codes)
-    CUtensorMap maps[4];        // TMA descriptors: p0, p1, p2, rhs
+    vof::J2Tables j2;           // of p0, p1, p2, rhs
     // convergent modes (VOF_MODE_MIXED / VOF_MODE_FP64)
     int conv;                   // nonzero in those modes
     double* p64;                // FP64 pressure (padded layout); p0 holds its FP32 copy
@@ -362,17 +362,15 @@ int vof_create(const vof_params* p, void* stream, vof_ctx** out) {
     c->b.vs = c->fields[VOF_FIELD_VSTAR - 1];
     c->b.ws = c->fields[VOF_FIELD_WSTAR - 1];
     c->b.rhs = c->fields[VOF_FIELD_RHS - 1];
-    c->b.maps = c->maps;
+    c->b.j2 = &c->j2;
     c->b.status = c->d_status;
     c->p_parity = 0;
     {
-        const float* mapped[4] = {c->b.p0, c->b.p1, c->b.p2, c->b.rhs};
-        for (int q = 0; q < 4; ++q) {
-            if ((e = vof::jacobi_tb_maps(c->g, mapped[q], &c->maps[q])) != cudaSuccess) {
-                c->last_cuda_error = (int)e;
-                free_ctx(c);
-                return VOF_E_UNSUPPORTED;
-            }
+        float* const mapped[4] = {c->b.p0, c->b.p1, c->b.p2, c->b.rhs};
+        if ((e = vof::jacobi_two_prepare(c->g, mapped, &c->j2, c->stream)) != cudaSuccess) {
+            c->last_cuda_error = (int)e;
+            free_ctx(c);
+            return VOF_E_UNSUPPORTED;
         }
     }
 

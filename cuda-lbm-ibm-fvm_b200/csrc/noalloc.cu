@@ -25,7 +25,7 @@
 #include <mutex>
 
 #include "../../include/vof.h"
-#include "jacobi_tb.h"
+#include "jacobi_two.h"
 #include "plain_step.h"
 #include "tma.cuh"
 
@@ -126,10 +126,9 @@ extern "C" int vof_step_noalloc(const vof_params* prm, float* F, float* u, float
     if (e == cudaSuccess) e = vof::plain_density_pairs_on(&g, tail, s);
     if (e != cudaSuccess) return VOF_E_CUDA;
 
-    CUtensorMap maps[4];
-    const float* mapped[4] = {f[8], f[9], f[10], f[7]};
-    for (int q = 0; q < 4; ++q)
-        if (vof::jacobi_tb_maps(g, mapped[q], &maps[q]) != cudaSuccess) return VOF_E_UNSUPPORTED;
+    vof::J2Tables j2;
+    float* const mapped[4] = {f[8], f[9], f[10], f[7]};
+    if (vof::jacobi_two_prepare(g, mapped, &j2, s) != cudaSuccess) return VOF_E_UNSUPPORTED;
 
     vof::PlainBuffers b;
     memset(&b, 0, sizeof(b));
@@ -144,7 +143,7 @@ extern "C" int vof_step_noalloc(const vof_params* prm, float* F, float* u, float
     b.p0 = f[8];
     b.p1 = f[9];
     b.p2 = f[10];
-    b.maps = maps;
+    b.j2 = &j2;
     b.status = status;
     int parity = 0;
     e = vof::plain_step(g, b, istep, prm->jacobi_iters, &parity, s, nullptr);

@@ -14,8 +14,8 @@
 //                  two cells per thread (k_predict: one; VOF_PREDICT=1)
 //   k_rhs4         the rhs expression of solve_p_jacobi_kernel voftrial1.cu:418-422
 //                  four cells per thread (k_rhs: one, marching z; VOF_RHS=1)
-//   k_jacobi_peel  (jacobi_tb.cu) one solve_p_jacobi_kernel sweep per launch,  voftrial1.cu:401-439
-//                  two cells per thread (alternatives selected by VOF_JACOBI, below)
+//   k_jacobi_two   (jacobi_two.cu) two solve_p_jacobi_kernel sweeps per launch,  voftrial1.cu:401-439
+//                  four cells per thread (an odd one: k_jacobi_peel, jacobi.cu)
 //   k_correct4     update_{u,v,w}_kernel + apply_bc_velocity   voftrial1.cu:441-493, 959-1051, 1107-1120
 //                  four cells per thread (k_correct: one; VOF_CORRECT=1)
 //   k_fct<AXIS,FINAL>  (fct_sweep.cu) fct_{x,y,z}_sweep_stage1..4, and on
@@ -23,7 +23,8 @@
 #include "plain_step.h"
 
 #include "fct_sweep.h"
-#include "jacobi_tb.h"
+#include "jacobi.h"
+#include "jacobi_two.h"
 
 #include <cuda_runtime.h>
 #include <stdlib.h>
@@ -668,7 +669,8 @@ __global__ void __launch_bounds__(256, 4) k_correct4(Geom g, const float* __rest
 cudaError_t plain_configure(int max_line) {
     (void)max_line;
     cudaError_t e = fct_configure();
-    return e == cudaSuccess ? jacobi_tb_configure() : e;
+    if (e == cudaSuccess) e = jacobi_configure();
+    return e == cudaSuccess ? jacobi_two_configure() : e;
 }
 
 cudaError_t plain_density_pairs(Geom* g) {
@@ -707,106 +709,22 @@ bool plain_supported(const Geom& g) {
            fct_smem_bytes(2, g.nz) <= fct_smem_limit();
 }
 
-// Sweeps fused per Jacobi launch (1 .. JACOBI_TB_MAX).
-#ifndef VOF_JACOBI_T
-#define VOF_JACOBI_T 2
-#endif
-constexpr int JACOBI_T = VOF_JACOBI_T;
-static_assert(JACOBI_T >= 1 && JACOBI_T <= JACOBI_TB_MAX, "VOF_JACOBI_T out of range");
-
-// Launches for `iters` sweeps: ceil(iters / JACOBI_T), except that a single
-// blocked launch cannot end in the buffer it reads, so iters == JACOBI_T
-// (even) runs as single sweeps.
-// Jacobi kernels.  One sweep per launch: two cells per thread with the
-// plane cases peeled out of the z march (k_jacobi_peel, the default), the
-// same without the peeling (k_jacobi_pairs), with its own column's loads
-// copied several planes ahead (k_jacobi_ring), fed by bulk copies of whole
-// rows (k_jacobi_bulk), with four cells per thread (k_jacobi_quad), with one
-// cell per thread (k_jacobi_col), or through TMA tiles (k_jacobi_tb, one
-// sweep: tb1).  Several sweeps per launch: two cells per thread, two sweeps
-// (k_jacobi_pairs2; an odd count starts with one single sweep), or JACOBI_T
-// temporally blocked sweeps through TMA (k_jacobi_tb).
-// VOF_JACOBI=peel|pairs|ring|bulk|quad|col|tb1|pairs2|tb forces one.  All
-// give the same bits.
-enum { JACOBI_PAIRS = 0, JACOBI_COL = 1, JACOBI_TB = 2, JACOBI_PAIRS2 = 3, JACOBI_RING = 4, JACOBI_PEEL = 5, JACOBI_TB1 = 6, JACOBI_BULK = 7, JACOBI_QUAD = 8 };
-static int jacobi_kind(const Geom& g) {
-    static int forced = -2;
-    if (forced == -2) {
+// Two sweeps per launch (k_jacobi_two), an odd count starting with one single
+// sweep (k_jacobi_peel), on grids of at least 2^19 cells; below, its march is
+// too short to pay for the halo (64^3: 30 steps 4.56 against 4.45 ms, 32^3
+// 1.65 against 1.59).  VOF_JACOBI=peel / two force either (same bits).
+static bool jacobi_two(const Geom& g, int iters) {
+    static int forced = -1;
+    if (forced < 0) {
         const char* v = getenv("VOF_JACOBI");
-        forced = -1;
-        if (v && !strcmp(v, "pairs")) forced = JACOBI_PAIRS;
-        if (v && !strcmp(v, "col")) forced = JACOBI_COL;
-        if (v && !strcmp(v, "tb")) forced = JACOBI_TB;
-        if (v && !strcmp(v, "pairs2")) forced = JACOBI_PAIRS2;
-        if (v && !strcmp(v, "ring")) forced = JACOBI_RING;
-        if (v && !strcmp(v, "peel")) forced = JACOBI_PEEL;
-        if (v && !strcmp(v, "tb1")) forced = JACOBI_TB1;
-        if (v && !strcmp(v, "bulk")) forced = JACOBI_BULK;
-        if (v && !strcmp(v, "quad")) forced = JACOBI_QUAD;
+        forced = v && !strcmp(v, "peel") ? 1 : v && !strcmp(v, "two") ? 2 : 0;
     }
-    const int k = forced >= 0 ? forced : JACOBI_PEEL;
-    if (k == JACOBI_BULK && !jacobi_bulk_supported(g)) return JACOBI_PAIRS;
-    return (k == JACOBI_PAIRS2 && !jacobi_pairs2_supported(g)) ? JACOBI_PAIRS : k;
-}
-// The peeled kernel marches z downwards on every second sweep when the
-// three buffers the sweeps touch (two pressures and rhs) are at most 1.25x
-// the L2: a sweep then starts on the planes the previous one touched last,
-// which are still in L2, instead of on the ones touched first, which a
-// cyclic march has evicted.  Measured on a B200: 200^3 (110 MB) 4 % faster
-// sweeps, 128^3 (all in L2) unchanged, 256^3 (230 MB) 1 % slower.
-// VOF_JACOBI_ALT=0 / 1 forces it off / on.
-static bool jacobi_alternate(const Geom& g) {
-    static int forced = -2;
-    static long long l2 = 0;
-    if (forced == -2) {
-        const char* v = getenv("VOF_JACOBI_ALT");
-        forced = v ? (atoi(v) != 0 ? 1 : 0) : -1;
-        int dev = 0, b = 0;
-        if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&b, cudaDevAttrL2CacheSize, dev) == cudaSuccess)
-            l2 = b;
-    }
-    if (forced >= 0) return forced == 1;
-    const long long bytes = 3LL * g.plane * (g.nz + 2) * (long long)sizeof(float);
-    return l2 > 0 && 4 * bytes <= 5 * l2;
+    // (a launch cannot end in the buffer it reads, where two sweeps have to end)
+    if (iters <= 2 || forced == 1) return false;
+    return forced == 2 || (long long)g.nx * g.ny * g.nz >= 1 << 19;
 }
 
-static bool jacobi_streaming(const Geom& g) {
-    const int k = jacobi_kind(g);
-    return k == JACOBI_PAIRS || k == JACOBI_COL || k == JACOBI_RING || k == JACOBI_PEEL || k == JACOBI_BULK ||
-           k == JACOBI_QUAD;
-}
-static int jacobi_per_launch(const Geom& g) {
-    const int k = jacobi_kind(g);
-    return k == JACOBI_PAIRS2 ? 2 : k == JACOBI_TB1 ? 1 : JACOBI_T;
-}
-
-static int jacobi_launches(const Geom& g, int iters) {
-    if (jacobi_streaming(g)) return iters;
-    const int T = jacobi_per_launch(g);
-    const int L = (iters + T - 1) / T;
-    return (L == 1 && iters % 2 == 0) ? iters : L;
-}
-
-// Buffer sequence for L blocked launches taking the pressure from physical
-// buffer `src` to `dst` (0/1: the two buffers the reference ping-pongs; 2: a
-// scratch buffer), consecutive buffers distinct.  Returns false when no such
-// sequence exists (L == 1 with src == dst).
-static bool plan_buffers(int src, int dst, int L, int* seq) {
-    if (L == 0) return src == dst;
-    if (L == 1 && src == dst) return false;
-    seq[0] = src;
-    seq[L] = dst;
-    for (int q = L - 1; q >= 1; --q) {
-        int c = 2;
-        if (c == seq[q + 1]) c = (seq[q + 1] == 0) ? 1 : 0;
-        if (q == 1 && c == src) {
-            for (int t = 0; t < 3; ++t)
-                if (t != src && t != seq[2]) c = t;
-        }
-        seq[q] = c;
-    }
-    return true;
-}
+static int jacobi_launches(const Geom& g, int iters) { return jacobi_two(g, iters) ? (iters + 1) / 2 : iters; }
 
 int plain_kernels_per_step(const Geom& g, int jacobi_iters) {
     return 1 + (g.csf ? 3 : 0) + 1 + jacobi_launches(g, jacobi_iters) + 1 + 3;
@@ -941,57 +859,31 @@ cudaError_t plain_back(const Geom& g, const PlainBuffers& b, int istep, const fl
 cudaError_t plain_pressure(const Geom& g, const PlainBuffers& b, int jacobi_iters, int* p_parity, cudaStream_t s) {
     cudaError_t e;
 
-    // Jacobi (voftrial1.cu:1371-1375): one streaming sweep per launch on
-    // small grids, else JACOBI_T blocked sweeps per launch.  The
-    // reference ping-pongs p <-> pt once per sweep, so after N sweeps its
-    // pressure sits in the buffer it started in when N is even and in the
-    // other one when N is odd; the launches route through the scratch
-    // buffer so the result lands in that same buffer (which keeps the
-    // reference's ghost entries in a download).
+    // Jacobi (voftrial1.cu:1371-1375).  The reference ping-pongs p <-> pt once
+    // per sweep, so after N sweeps its pressure sits in the buffer it started
+    // in when N is even and in the other one when N is odd; the launches end in
+    // that same buffer (which keeps the reference's ghost entries in a
+    // download), through the scratch buffer first when their number is of the
+    // other parity.
     float* pbuf[3] = {b.p0, b.p1, b.p2};
     const int src = *p_parity, dst = src ^ (jacobi_iters & 1);
-    const int T = jacobi_per_launch(g);
-    const int L = (jacobi_iters + T - 1) / T;
-    int seq[64];
-    if (jacobi_kind(g) == JACOBI_PAIRS2 && L <= 62 && plan_buffers(src, dst, L, seq)) {
-        // an odd count starts with one single sweep
+    int cur = src;
+    if (jacobi_two(g, jacobi_iters)) {
+        const int L = jacobi_launches(g, jacobi_iters);
+        const bool detour = (L & 1) != (src != dst);
         for (int q = 0; q < L; ++q) {
-            const bool single = q == 0 && (jacobi_iters & 1);
-            e = single ? jacobi_pairs_launch(g, pbuf[seq[q]], b.rhs, pbuf[seq[q + 1]], s)
-                       : jacobi_pairs2_launch(g, pbuf[seq[q]], b.rhs, pbuf[seq[q + 1]], s);
+            const int left = L - 1 - q;  // launches after this one, each between the two buffers
+            const int to = detour && q == 0 ? 2 : dst ^ (left & 1);
+            if (q == 0 && (jacobi_iters & 1))
+                e = jacobi_peel_launch(g, pbuf[cur], b.rhs, pbuf[to], s);
+            else
+                e = jacobi_two_launch(g, *b.j2, cur, pbuf[cur], pbuf[to], b.status, s);
             if (e != cudaSuccess) return e;
-        }
-    } else if (jacobi_streaming(g) || jacobi_kind(g) == JACOBI_PAIRS2) {
-        int cur = src;
-        const int kind = jacobi_kind(g);
-        const bool alt = kind == JACOBI_PEEL && jacobi_alternate(g);
-        for (int it = 0; it < jacobi_iters; ++it) {
-            e = kind == JACOBI_COL    ? jacobi_col_launch(g, pbuf[cur], b.rhs, pbuf[cur ^ 1], s)
-                : kind == JACOBI_RING ? jacobi_ring_launch(g, pbuf[cur], b.rhs, pbuf[cur ^ 1], s)
-                : kind == JACOBI_PEEL ? jacobi_peel_launch(g, pbuf[cur], b.rhs, pbuf[cur ^ 1], s,
-                                                           alt && (it & 1))
-                : kind == JACOBI_BULK ? jacobi_bulk_launch(g, pbuf[cur], b.rhs, pbuf[cur ^ 1], b.status, s)
-                : kind == JACOBI_QUAD ? jacobi_quad_launch(g, pbuf[cur], b.rhs, pbuf[cur ^ 1], s)
-                                      : jacobi_pairs_launch(g, pbuf[cur], b.rhs, pbuf[cur ^ 1], s);
-            if (e != cudaSuccess) return e;
-            cur ^= 1;
-        }
-    } else if (L > 62 || !plan_buffers(src, dst, L, seq)) {
-        // fall back to one sweep per launch: a plain ping-pong always works
-        int cur = src;
-        for (int it = 0; it < jacobi_iters; ++it) {
-            if ((e = jacobi_tb_launch(g, 1, b.maps[cur], b.maps[3], pbuf[cur ^ 1], b.status, s)) != cudaSuccess)
-                return e;
-            cur ^= 1;
+            cur = to;
         }
     } else {
-        const int T1 = jacobi_per_launch(g);
-        for (int q = 0; q < L; ++q) {
-            const int T = (q == 0 && jacobi_iters % T1) ? jacobi_iters % T1 : T1;
-            if ((e = jacobi_tb_launch(g, T, b.maps[seq[q]], b.maps[3], pbuf[seq[q + 1]], b.status, s)) !=
-                cudaSuccess)
-                return e;
-        }
+        for (int it = 0; it < jacobi_iters; ++it, cur ^= 1)
+            if ((e = jacobi_peel_launch(g, pbuf[cur], b.rhs, pbuf[cur ^ 1], s)) != cudaSuccess) return e;
     }
     *p_parity = dst;
     return cudaSuccess;

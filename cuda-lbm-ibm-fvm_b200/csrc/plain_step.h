@@ -1,8 +1,8 @@
 // plain_step.h -- host-side interface of the FP32 drop-in step kernels.
 #pragma once
-#include <cuda.h>
 #include <cuda_runtime.h>
 
+#include "jacobi_two.h"
 #include "vof_device.cuh"
 
 namespace vof {
@@ -20,7 +20,7 @@ struct PlainBuffers {
     float* p0;   // Jacobi ping-pong pair (DeviceFields::p / ::pt)
     float* p1;
     float* p2;   // scratch pressure buffer for the blocked sweeps
-    const CUtensorMap* maps;  // TMA descriptors of p0, p1, p2, rhs (in that order)
+    const J2Tables* j2;       // of p0, p1, p2 and rhs (jacobi_two_prepare)
     int* status;              // device status word (DEV_* codes, tma.cuh)
     float* csf[4];            // g.csf: interface normal x, y, z and curvature per cell; else null
 };

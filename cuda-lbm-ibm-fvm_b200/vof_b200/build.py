@@ -32,7 +32,8 @@ COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-I" + str(IN
 SOURCES = {
     "plain_step.cu": ["-fmad=false", "-DVOF_FMAD_FALSE"],
     "fct_sweep.cu": ["-fmad=false", "-DVOF_FMAD_FALSE"],
-    "jacobi_tb.cu": ["-fmad=false", "-DVOF_FMAD_FALSE"],
+    "jacobi.cu": ["-fmad=false", "-DVOF_FMAD_FALSE"],
+    "jacobi_two.cu": ["-fmad=false", "-DVOF_FMAD_FALSE"],
     "adjoint.cu": ["-fmad=false", "-DVOF_FMAD_FALSE"],
     "tma_host.cu": [],
     "mg_solve.cu": [],
@@ -42,7 +43,7 @@ SOURCES = {
     "noalloc.cu": [],
     "apply_bc.cu": [],
 }
-HEADERS = ["vof_device.cuh", "tma.cuh", "plain_step.h", "fct_sweep.h", "fct_line.cuh", "jacobi_tb.h", "mg_solve.h", "spectral.h", "pdl.cuh",
+HEADERS = ["vof_device.cuh", "tma.cuh", "plain_step.h", "fct_sweep.h", "fct_line.cuh", "jacobi.h", "jacobi_two.h", "mg_solve.h", "spectral.h", "pdl.cuh",
            "reduce.h", "adjoint.h", "apply_bc.h"]
 
 
