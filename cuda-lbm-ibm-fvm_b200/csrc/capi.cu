@@ -15,6 +15,7 @@
 #include "jacobi_two.h"
 #include "adjoint.h"
 #include "apply_bc.h"
+#include "host_pull.h"
 #include "mg_solve.h"
 #include "plain_step.h"
 #include "reduce.h"
@@ -50,6 +51,7 @@ struct vof_ctx {
     vof::MgStats stats;         // of the last pressure solve
     vof::AdjEngine* adj;        // adjoint engine (vof_forward_record / vof_backward), or null
     int adj_policy;             // VOF_ADJ_* for the next vof_forward_record
+    vof::HostPull pull;         // of vof_adjoint_download
     cudaGraphExec_t graph[3][2];  // [istep % 3][p parity at step start]
     int last_cuda_error;
     size_t bytes;
@@ -130,6 +132,7 @@ void free_ctx(vof_ctx* c) {
         vof::adj_destroy(c->adj);
         delete c->adj;
     }
+    vof::host_pull_destroy(&c->pull);
     if (c->cap_stream) cudaStreamDestroy(c->cap_stream);
     delete c;
 }
@@ -140,16 +143,18 @@ void free_ctx(vof_ctx* c) {
 // contiguous cudaMemcpyAsync through the context's staging buffer, and this
 // kernel repacks it: a row of (nx+2) floats is 808 bytes at 200^3, and
 // row-by-row host copies of that size run far below the link's bandwidth.
-__global__ void __launch_bounds__(256) k_repack(const float* __restrict__ src, int spitch, float* __restrict__ dst,
+template <typename T>
+__global__ void __launch_bounds__(256) k_repack(const T* __restrict__ src, int spitch, T* __restrict__ dst,
                                                 int dpitch, int width, int rows) {
     for (int r = blockIdx.x * 8 + threadIdx.y; r < rows; r += gridDim.x * 8) {
-        const float* a = src + (size_t)r * spitch;
-        float* b = dst + (size_t)r * dpitch;
+        const T* a = src + (size_t)r * spitch;
+        T* b = dst + (size_t)r * dpitch;
         for (int i = threadIdx.x; i < width; i += 32) b[i] = a[i];
     }
 }
 
-cudaError_t repack(const float* src, int spitch, float* dst, int dpitch, int width, int rows, cudaStream_t s) {
+template <typename T>
+cudaError_t repack(const T* src, int spitch, T* dst, int dpitch, int width, int rows, cudaStream_t s) {
     int blocks = (rows + 7) / 8;
     if (blocks > 148 * 16) blocks = 148 * 16;
     k_repack<<<blocks, dim3(32, 8), 0, s>>>(src, spitch, dst, dpitch, width, rows);
@@ -413,7 +418,7 @@ int vof_upload(vof_ctx* ctx, int field, const float* src, int src_is_device) {
                             ctx->stream);
         from = ctx->stage;
     }
-    if (e == cudaSuccess) e = repack(from, g.nx + 2, dst, g.px, g.nx + 2, rows, ctx->stream);
+    if (e == cudaSuccess) e = repack<float>(from, g.nx + 2, dst, g.px, g.nx + 2, rows, ctx->stream);
     if (e == cudaSuccess && ctx->conv && field == VOF_FIELD_P) e = vof::mg_widen(g, ctx->mg, dst, ctx->p64, ctx->stream);
     return e == cudaSuccess ? VOF_OK : fail_cuda(ctx, e);
 }
@@ -425,7 +430,7 @@ int vof_download(vof_ctx* ctx, int field, float* dst, int dst_is_device) {
     DeviceGuard dg(ctx->device);
     const Geom& g = ctx->g;
     const int rows = (g.ny + 2) * (g.nz + 2);
-    cudaError_t e = repack(src, g.px, dst_is_device ? dst : ctx->stage, g.nx + 2, g.nx + 2, rows, ctx->stream);
+    cudaError_t e = repack<float>(src, g.px, dst_is_device ? dst : ctx->stage, g.nx + 2, g.nx + 2, rows, ctx->stream);
     if (e == cudaSuccess && !dst_is_device) {  // the repacked field in one contiguous copy
         e = cudaMemcpyAsync(dst, ctx->stage, (size_t)ctx->prm.nTot * sizeof(float), cudaMemcpyDeviceToHost,
                             ctx->stream);
@@ -441,7 +446,7 @@ int vof_get_planes(vof_ctx* ctx, int field, int k0, int nk, float* dst, int dst_
     DeviceGuard dg(ctx->device);
     const Geom& g = ctx->g;
     const int rows = (g.ny + 2) * nk;
-    cudaError_t e = repack(src + (size_t)k0 * g.plane, g.px, dst_is_device ? dst : ctx->stage, g.nx + 2, g.nx + 2,
+    cudaError_t e = repack<float>(src + (size_t)k0 * g.plane, g.px, dst_is_device ? dst : ctx->stage, g.nx + 2, g.nx + 2,
                            rows, ctx->stream);
     if (e == cudaSuccess && !dst_is_device) {
         e = cudaMemcpyAsync(dst, ctx->stage, (size_t)rows * (g.nx + 2) * sizeof(float), cudaMemcpyDeviceToHost,
@@ -466,7 +471,7 @@ int vof_put_planes(vof_ctx* ctx, int field, int k0, int nk, const float* src, in
                             ctx->stream);
         from = ctx->stage;
     }
-    if (e == cudaSuccess) e = repack(from, g.nx + 2, dst + (size_t)k0 * g.plane, g.px, g.nx + 2, rows, ctx->stream);
+    if (e == cudaSuccess) e = repack<float>(from, g.nx + 2, dst + (size_t)k0 * g.plane, g.px, g.nx + 2, rows, ctx->stream);
     return e == cudaSuccess ? VOF_OK : fail_cuda(ctx, e);
 }
 
@@ -768,10 +773,11 @@ int vof_adjoint_download(vof_ctx* ctx, int field, double* dst) {
     const vof::AdjEngine* A = ctx->adj;
     const double* src[5] = {A->lF, A->lu, A->lv, A->lw, A->lp[A->lp_cur]};
     const Geom& g = ctx->g;
-    const size_t w = (size_t)(g.nx + 2) * sizeof(double);
-    cudaError_t e = cudaMemcpy2DAsync(dst, w, src[field], (size_t)g.px * sizeof(double), w,
-                                      (size_t)(g.ny + 2) * (g.nz + 2), cudaMemcpyDeviceToHost, ctx->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    // repacked on the device into a field that the reverse pass clears before
+    // it uses it, then one contiguous copy
+    cudaError_t e = repack<double>(src[field], g.px, A->lus, g.nx + 2, g.nx + 2, (g.ny + 2) * (g.nz + 2), ctx->stream);
+    if (e == cudaSuccess)
+        e = vof::host_pull(&ctx->pull, dst, A->lus, (size_t)ctx->prm.nTot * sizeof(double), ctx->stream);
     return e == cudaSuccess ? VOF_OK : fail_cuda(ctx, e);
 }
 

@@ -1,0 +1,103 @@
+// host_pull.cu -- device to host copies into memory of any kind.
+//
+// A copy into pageable memory goes through the driver's staging buffer: one
+// thread moves it on, and takes the page faults of memory that was never
+// touched, which a fresh numpy array is.  Measured on a B200's host, 25 MB
+// arrays: 3.4 ms each (7 GB/s).  Here several threads own a slice each, bring
+// it in over the link in chunks (two in flight) and move those on side by side.
+#include "host_pull.h"
+
+#include <string.h>
+
+#include <atomic>
+#include <system_error>
+#include <thread>
+
+namespace vof {
+
+static cudaError_t make(HostPull* h) {
+    cudaError_t e;
+    if ((e = cudaMallocHost((void**)&h->pinned, PULL_THREADS * 2 * PULL_CHUNK)) != cudaSuccess) {
+        h->pinned = nullptr;
+        return e;
+    }
+    if ((e = cudaEventCreateWithFlags(&h->ready, cudaEventDisableTiming)) != cudaSuccess) return e;
+    for (int t = 0; t < PULL_THREADS; ++t) {
+        if ((e = cudaStreamCreateWithFlags(&h->stream[t], cudaStreamNonBlocking)) != cudaSuccess) return e;
+        for (int b = 0; b < 2; ++b)
+            if ((e = cudaEventCreateWithFlags(&h->done[t][b], cudaEventDisableTiming)) != cudaSuccess) return e;
+    }
+    h->made = true;
+    return cudaSuccess;
+}
+
+void host_pull_destroy(HostPull* h) {
+    if (h->pinned) cudaFreeHost(h->pinned);
+    if (h->ready) cudaEventDestroy(h->ready);
+    for (int t = 0; t < PULL_THREADS; ++t) {
+        if (h->stream[t]) cudaStreamDestroy(h->stream[t]);
+        for (int b = 0; b < 2; ++b)
+            if (h->done[t][b]) cudaEventDestroy(h->done[t][b]);
+    }
+    *h = HostPull{};
+}
+
+// Slice [at, end) of the copy by thread t.
+static cudaError_t slice(HostPull* h, int t, char* dst, const char* src, size_t at, size_t end) {
+    cudaError_t e = cudaStreamWaitEvent(h->stream[t], h->ready, 0);
+    char* const buf[2] = {h->pinned + (2 * t) * PULL_CHUNK, h->pinned + (2 * t + 1) * PULL_CHUNK};
+    auto bytes = [&](size_t a) { return end - a < PULL_CHUNK ? end - a : PULL_CHUNK; };
+    auto issue = [&](size_t a, int b) {
+        cudaError_t r = cudaMemcpyAsync(buf[b], src + a, bytes(a), cudaMemcpyDeviceToHost, h->stream[t]);
+        return r == cudaSuccess ? cudaEventRecord(h->done[t][b], h->stream[t]) : r;
+    };
+    if (e == cudaSuccess && at < end) e = issue(at, 0);
+    for (int b = 0; at < end && e == cudaSuccess; b ^= 1) {
+        const size_t n = bytes(at);
+        if (at + n < end) e = issue(at + n, b ^ 1);
+        if (e == cudaSuccess) e = cudaEventSynchronize(h->done[t][b]);
+        if (e == cudaSuccess) memcpy(dst + at, buf[b], n);
+        at += n;
+    }
+    if (e != cudaSuccess) cudaStreamSynchronize(h->stream[t]);  // no copy stays in flight
+    return e;
+}
+
+cudaError_t host_pull(HostPull* h, void* dst, const void* src, size_t bytes, cudaStream_t s) {
+    cudaError_t e = cudaSuccess;
+    cudaPointerAttributes at;
+    const bool pageable = cudaPointerGetAttributes(&at, dst) != cudaSuccess || at.type == cudaMemoryTypeUnregistered;
+    cudaGetLastError();
+    if (bytes >= (4u << 20) && pageable && !h->made && make(h) != cudaSuccess) {
+        cudaGetLastError();
+        host_pull_destroy(h);  // (no pinned memory to be had: the plain copy)
+    }
+    if (bytes < (4u << 20) || !pageable || !h->made) {
+        e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s);
+        return e == cudaSuccess ? cudaStreamSynchronize(s) : e;
+    }
+    int device = 0;
+    if ((e = cudaEventRecord(h->ready, s)) != cudaSuccess || (e = cudaGetDevice(&device)) != cudaSuccess) return e;
+    std::atomic<int> err{cudaSuccess};
+    const size_t chunks = (bytes + PULL_CHUNK - 1) / PULL_CHUNK;
+    auto work = [&](int t) {
+        const size_t a = chunks * t / PULL_THREADS * PULL_CHUNK, b = chunks * (t + 1) / PULL_THREADS * PULL_CHUNK;
+        cudaError_t r = cudaSetDevice(device);
+        if (r == cudaSuccess)
+            r = slice(h, t, static_cast<char*>(dst), static_cast<const char*>(src), a, b < bytes ? b : bytes);
+        if (r != cudaSuccess) err.store(r);
+    };
+    std::thread th[PULL_THREADS];
+    int started = 1;
+    try {
+        for (; started < PULL_THREADS; ++started) th[started] = std::thread(work, started);
+    } catch (const std::system_error&) {
+        // (no more threads: their slices below)
+    }
+    work(0);
+    for (int t = started; t < PULL_THREADS; ++t) work(t);
+    for (int t = 1; t < started; ++t) th[t].join();
+    return (cudaError_t)err.load();
+}
+
+}  // namespace vof

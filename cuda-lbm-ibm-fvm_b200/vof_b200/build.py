@@ -41,9 +41,10 @@ SOURCES = {
     "reduce.cu": [],
     "capi.cu": [],
     "noalloc.cu": [],
+    "host_pull.cu": [],
     "apply_bc.cu": [],
 }
-HEADERS = ["vof_device.cuh", "tma.cuh", "plain_step.h", "fct_sweep.h", "fct_line.cuh", "jacobi.h", "jacobi_two.h", "mg_solve.h", "spectral.h", "pdl.cuh",
+HEADERS = ["vof_device.cuh", "tma.cuh", "plain_step.h", "fct_sweep.h", "fct_line.cuh", "jacobi.h", "jacobi_two.h", "host_pull.h", "mg_solve.h", "spectral.h", "pdl.cuh",
            "reduce.h", "adjoint.h", "apply_bc.h"]
 
 
