@@ -1603,10 +1603,8 @@ cudaError_t recompute_step(AdjEngine& e, const AdjState& x, int istep, StepData*
     if ((r = plain_correct(g, e.wb, pafter, s)) != cudaSuccess) return r;
     const int* dirs = sweep_order(istep);
     const float* velof[3] = {e.wb.u, e.wb.v, e.wb.w};
-    if ((r = copy_field(e.Fin1, x.f[0], e.elems, s)) != cudaSuccess ||
-        (r = fct_launch(g, dirs[0], false, e.Fin1, velof[dirs[0]], s)) != cudaSuccess ||
-        (r = copy_field(e.Fin2, e.Fin1, e.elems, s)) != cudaSuccess ||
-        (r = fct_launch(g, dirs[1], false, e.Fin2, velof[dirs[1]], s)) != cudaSuccess)
+    if ((r = fct_launch_to(g, dirs[0], false, x.f[0], e.Fin1, velof[dirs[0]], s)) != cudaSuccess ||
+        (r = fct_launch_to(g, dirs[1], false, e.Fin1, e.Fin2, velof[dirs[1]], s)) != cudaSuccess)
         return r;
     *d = StepData{x.f[0], x.f[1], x.f[2], x.f[3], e.wb.us, e.wb.vs, e.wb.ws, pafter,
                   {velof[0], velof[1], velof[2]}, {x.f[0], e.Fin1, e.Fin2}};

@@ -379,8 +379,7 @@ int vof_create(const vof_params* p, void* stream, vof_ctx** out) {
         }
     }
 
-    const int maxn = p->nx > p->ny ? (p->nx > p->nz ? p->nx : p->nz) : (p->ny > p->nz ? p->ny : p->nz);
-    if ((e = vof::plain_configure(maxn)) != cudaSuccess || (e = vof::plain_density_pairs(&c->g)) != cudaSuccess ||
+    if ((e = vof::plain_configure()) != cudaSuccess || (e = vof::plain_density_pairs(&c->g)) != cudaSuccess ||
         (e = cudaStreamCreateWithFlags(&c->cap_stream, cudaStreamNonBlocking)) != cudaSuccess ||
         (e = cudaStreamSynchronize(c->stream)) != cudaSuccess) {
         c->last_cuda_error = (int)e;

@@ -50,7 +50,7 @@ int arena_base(float** out) {
     if (!g_base[dev]) {
         void* p = nullptr;
         if (cudaGetSymbolAddress(&p, g_arena) != cudaSuccess) return VOF_E_CUDA;
-        if (vof::plain_configure(0) != cudaSuccess) return VOF_E_CUDA;
+        if (vof::plain_configure() != cudaSuccess) return VOF_E_CUDA;
         g_base[dev] = static_cast<float*>(p);
     }
     *out = g_base[dev];

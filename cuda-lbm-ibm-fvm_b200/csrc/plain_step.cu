@@ -666,10 +666,8 @@ __global__ void __launch_bounds__(256, 4) k_correct4(Geom g, const float* __rest
 // ---------------------------------------------------------------------------
 // Host launchers
 // ---------------------------------------------------------------------------
-cudaError_t plain_configure(int max_line) {
-    (void)max_line;
-    cudaError_t e = fct_configure();
-    if (e == cudaSuccess) e = jacobi_configure();
+cudaError_t plain_configure() {
+    const cudaError_t e = jacobi_configure();
     return e == cudaSuccess ? jacobi_two_configure() : e;
 }
 
@@ -705,8 +703,7 @@ cudaError_t plain_density_pairs_on(Geom* g, float* dev6, cudaStream_t s) {
 }
 
 bool plain_supported(const Geom& g) {
-    return fct_smem_bytes(0, g.nx) <= fct_smem_limit() && fct_smem_bytes(1, g.ny) <= fct_smem_limit() &&
-           fct_smem_bytes(2, g.nz) <= fct_smem_limit();
+    return fct_supported(g.nx) && fct_supported(g.ny) && fct_supported(g.nz);
 }
 
 // Two sweeps per launch (k_jacobi_two), an odd count starting with one single
@@ -844,14 +841,12 @@ cudaError_t plain_back(const Geom& g, const PlainBuffers& b, int istep, const fl
     static const int order[3][3] = {{0, 1, 2}, {1, 2, 0}, {2, 0, 1}};
     float* s1 = (p == b.p0) ? b.p1 : b.p0;
     float* s2 = b.p2;
-    const bool oop = s1 && s2 && p != b.p2;
     const float* src[3] = {b.F, s1, s2};
     float* dst[3] = {s1, s2, b.F};
     for (int q = 0; q < 3; ++q) {
         const int axis = order[r][q];
         const float* vel = axis == 0 ? b.u : (axis == 1 ? b.v : b.w);
-        e = oop ? fct_launch_to(g, axis, q == 2, src[q], dst[q], vel, s) : fct_launch(g, axis, q == 2, b.F, vel, s);
-        if (e != cudaSuccess || (e = mark(ev, 5 + q, s)) != cudaSuccess) return e;
+        if ((e = fct_launch_to(g, axis, q == 2, src[q], dst[q], vel, s)) != cudaSuccess || (e = mark(ev, 5 + q, s)) != cudaSuccess) return e;
     }
     return cudaSuccess;
 }

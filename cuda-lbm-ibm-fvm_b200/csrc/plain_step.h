@@ -25,9 +25,8 @@ struct PlainBuffers {
     float* csf[4];            // g.csf: interface normal x, y, z and curvature per cell; else null
 };
 
-// Raise the dynamic shared-memory limit of the FCT kernels for lines of up to
-// max_line interior cells.  Call once per device before the first step.
-cudaError_t plain_configure(int max_line);
+// Query and configure the kernels.  Call once per device before the first step.
+cudaError_t plain_configure();
 
 // Fill g->rpair / g->qpair (the density pairs of pure cells and dt over
 // them) with device arithmetic.  Call once per context.
