@@ -154,7 +154,11 @@ __global__ void __launch_bounds__(256) k_predict(Geom g,
 // neighbours come from the lanes beside (a pair's left neighbour is the left
 // lane's second cell, its right neighbour the right lane's first), or from
 // memory at the ends of a warp and of a row.  Each cell's three updates keep
-// k_predict's expressions and operand order (same bits).
+// k_predict's expressions and operand order (same bits).  Bound by instruction
+// issue (209 thread instructions per cell, 70 % of the slots used): 77 -> 70
+// us at 200^3 and 507 -> 476 at 400^3 by predict_kchunk's shorter chunks, of
+// which blocks of 128 threads rather than 256 are 1 to 3 %.  Packed FP32 pairs
+// (f32x2) took 99 us at 200^3, one viscosity for two equal cells 76.6.
 // The pair's left (x-1 of the first cell) and right (x+1 of the second cell)
 // neighbours of a value held as a pair by every lane.
 __device__ __forceinline__ float left_of(float2 a, bool ldw, const float* __restrict__ p, int idl) {
@@ -166,7 +170,7 @@ __device__ __forceinline__ float right_of(float2 a, bool lde, const float* __res
     return lde ? __ldg(p + idr) : s;
 }
 
-__global__ void __launch_bounds__(256, 4) k_predict2(Geom g, const float* __restrict__ F,
+__global__ void __launch_bounds__(128, 8) k_predict2(Geom g, const float* __restrict__ F,
                                                      const float* __restrict__ u, const float* __restrict__ v,
                                                      const float* __restrict__ w, float* __restrict__ us,
                                                      float* __restrict__ vs, float* __restrict__ ws, int kchunk) {
@@ -401,6 +405,8 @@ __global__ void __launch_bounds__(256) k_rhs(Geom g,
 // and of the row above, w* of the plane and of the plane above -- and the
 // u* east of the quad's last cell from the next lane, or from memory at the
 // end of a warp or of a row.  k_rhs's expression and operand order per cell.
+// One rho / dt for a quad of equal F.  Bound by DRAM and its latency: 34.5 us
+// at 200^3 (4.6 TB/s), 223 at 400^3 (5.7).
 __device__ __forceinline__ float4 ld4g(const float* __restrict__ a) {
     return __ldg(reinterpret_cast<const float4*>(a));
 }
@@ -428,13 +434,20 @@ __global__ void __launch_bounds__(256) k_rhs4(Geom g, const float* __restrict__ 
     if (lde) ue = ue_m;
     if (!qa) return;
     const float rdt = __frcp_rn(g.dt);
-    float r[4];
+    float c[4], r[4];  // rho / dt
+    c[0] = div_rn_pre(rho_of(g, f4.x), g.dt, rdt);
+    const unsigned f0 = __float_as_uint(f4.x);
+    if (((__float_as_uint(f4.y) ^ f0) | (__float_as_uint(f4.z) ^ f0) | (__float_as_uint(f4.w) ^ f0)) == 0) {
+        c[1] = c[2] = c[3] = c[0];
+    } else {
+#pragma unroll
+        for (int e = 1; e < 4; ++e) c[e] = div_rn_pre(rho_of(g, el4(f4, e)), g.dt, rdt);
+    }
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-        const float rho = rho_of(g, el4(f4, e));
         const float uip = e == 3 ? ue : el4(u4, e + 1);
-        r[e] = div_rn_pre(rho, g.dt, rdt) * ((uip - el4(u4, e)) * g.dxi + (el4(vn4, e) - el4(v4, e)) * g.dyi +
-                                             (el4(wn4, e) - el4(w4, e)) * g.dzi);
+        r[e] = c[e] * ((uip - el4(u4, e)) * g.dxi + (el4(vn4, e) - el4(v4, e)) * g.dyi +
+                       (el4(wn4, e) - el4(w4, e)) * g.dzi);
     }
     if (i0 >= 1 && i0 + 3 <= g.nx) {
         *reinterpret_cast<float4*>(rhs + id) = make_float4(r[0], r[1], r[2], r[3]);
@@ -601,6 +614,11 @@ __global__ void __launch_bounds__(256) k_correct(Geom g,
 // start of a warp.  Each face keeps k_correct's expression and operand order
 // (same bits).  Quads without an edge cell store float4 words; the others go
 // through store_corrected cell by cell.
+//
+// Most quads lie in one phase: where the 13 values of F that enter are equal,
+// one density and one quotient serve the 12 faces (47 M warp instructions at
+// 200^3 without this, issue and latency together the bound; DRAM now: 69.7 ->
+// 59.5 us at 200^3, 4.3 TB/s; 460 -> 385 at 400^3, 5.3 TB/s).
 __global__ void __launch_bounds__(256, 4) k_correct4(Geom g, const float* __restrict__ F,
                                                   const float* __restrict__ us, const float* __restrict__ vs,
                                                   const float* __restrict__ ws, const float* __restrict__ p,
@@ -621,32 +639,43 @@ __global__ void __launch_bounds__(256, 4) k_correct4(Geom g, const float* __rest
     const float4 pc = ld4g(p + id), ps = ld4g(p + id - sy), pb = ld4g(p + id - sz);
     const float4 u4 = ld4g(us + id), v4 = ld4g(vs + id), w4 = ld4g(ws + id);
     const float fl = ldw ? __ldg(F + id - 1) : 0.0f, pl = ldw ? __ldg(p + id - 1) : 0.0f;
-    float rc[4] = {rho_of(g, fc.x), rho_of(g, fc.y), rho_of(g, fc.z), rho_of(g, fc.w)};
-    float rl = __shfl_up_sync(0xffffffffu, rc[3], 1), pw = __shfl_up_sync(0xffffffffu, pc.w, 1);
+    float fw = __shfl_up_sync(0xffffffffu, fc.w, 1), pw = __shfl_up_sync(0xffffffffu, pc.w, 1);
     if (ldw) {
-        rl = rho_of(g, fl);
+        fw = fl;
         pw = pl;
+    }
+    if (m == 0) fw = fc.x;  // (enters no face)
+    float qu[4], qv[4], qw[4];  // dt over the face densities
+    const unsigned f0 = __float_as_uint(fc.x);
+    unsigned differ = __float_as_uint(fw) ^ f0;
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+        differ |= (__float_as_uint(el4(fc, e)) ^ f0) | (__float_as_uint(el4(fs, e)) ^ f0) |
+                  (__float_as_uint(el4(fb, e)) ^ f0);
+    if (differ == 0) {
+        const float rho = rho_of(g, fc.x);
+        const float q0 = dt_over(g, 0.5f * (rho + rho));
+#pragma unroll
+        for (int e = 0; e < 4; ++e) qu[e] = qv[e] = qw[e] = q0;
+    } else {
+        float rw = rho_of(g, fw);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float rho_c = rho_of(g, el4(fc, e));
+            qu[e] = dt_over(g, 0.5f * (rho_c + rw));
+            qv[e] = dt_over(g, 0.5f * (rho_c + rho_of(g, el4(fs, e))));
+            qw[e] = dt_over(g, 0.5f * (rho_c + rho_of(g, el4(fb, e))));
+            rw = rho_c;
+        }
     }
     float un[4], vn[4], wn[4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-        const int i = i0 + e;
-        const float rho_c = rc[e], p_c = el4(pc, e);
-        un[e] = 0.0f;  // wall faces (i, j or k == 1) are 0
-        vn[e] = 0.0f;
-        wn[e] = 0.0f;
-        if (i >= 2) {
-            const float r = 0.5f * (rho_c + (e == 0 ? rl : rc[e - 1]));
-            un[e] = el4(u4, e) - dt_over(g, r) * (p_c - (e == 0 ? pw : el4(pc, e - 1))) * g.dxi;
-        }
-        if (j >= 2) {
-            const float r = 0.5f * (rho_c + rho_of(g, el4(fs, e)));
-            vn[e] = el4(v4, e) - dt_over(g, r) * (p_c - el4(ps, e)) * g.dyi;
-        }
-        if (k >= 2) {
-            const float r = 0.5f * (rho_c + rho_of(g, el4(fb, e)));
-            wn[e] = el4(w4, e) - dt_over(g, r) * (p_c - el4(pb, e)) * g.dzi;
-        }
+        const float p_c = el4(pc, e);
+        // wall faces (i, j or k == 1) are 0
+        un[e] = i0 + e >= 2 ? el4(u4, e) - qu[e] * (p_c - (e == 0 ? pw : el4(pc, e - 1))) * g.dxi : 0.0f;
+        vn[e] = j >= 2 ? el4(v4, e) - qv[e] * (p_c - el4(ps, e)) * g.dyi : 0.0f;
+        wn[e] = k >= 2 ? el4(w4, e) - qw[e] * (p_c - el4(pb, e)) * g.dzi : 0.0f;
     }
     if (!qa) return;
     const bool bulk = i0 >= 2 && i0 + 3 <= g.nx - 1 && j != 1 && j != g.ny && k != 1 && k != g.nz;
@@ -767,6 +796,28 @@ static int sm_count() {
     return n;
 }
 
+// Planes per block of k_predict2: the least estimate of its time in planes of
+// one resident block, waves of (kc + 1) planes each (the extra one for
+// the first window) and half a block for the uneven end.  Chunks as long as
+// one wave allows left the SMs with fewer blocks than others idle at the end:
+// (blocks of 256) 200^3 29 planes a block 76.8 us, 20 79.3, 16 73.0, 10 71.3,
+// 8 (chosen) 71.7, 7 69.3, 4 72.5; 400^3 50 planes 507, 20 (chosen) 480, 16
+// 482, 10 484, 7 495, 4 528; 128^3 8 planes 23.0, 4 (chosen) 22.2, 2 22.6.
+static int predict_kchunk(int nz, int bx, int wave) {
+    int best = 1;
+    double least = 1e30;
+    for (int kc = 1; kc <= nz; ++kc) {
+        const double waves = (double)bx * ((nz + kc - 1) / kc) / wave;
+        const double cost = ((waves > 1.0 ? waves : 1.0) + 0.6) * (kc + 1);
+        if (cost < least) {
+            least = cost;
+            best = kc;
+        }
+        if (waves < 0.5) break;
+    }
+    return best;
+}
+
 // 1: the one-cell kernel, 4: the four-cell kernel, else by size.
 static int env_kernel(const char* name) {
     const char* v = getenv(name);
@@ -785,9 +836,9 @@ cudaError_t plain_front(const Geom& g, const PlainBuffers& b, cudaStream_t s, cu
     if (pforced == 1) {
         k_predict<<<grid, blk, 0, s>>>(g, b.F, b.u, b.v, b.w, b.us, b.vs, b.ws, kchunk);
     } else {
-        const int bx = ((g.nx / 2 + 1) * g.ny + 255) / 256;
-        const int kc = wave_kchunk(g.nz, bx, 4 * sm_count());
-        k_predict2<<<dim3(bx, (g.nz + kc - 1) / kc), 256, 0, s>>>(g, b.F, b.u, b.v, b.w, b.us, b.vs, b.ws, kc);
+        const int bx = ((g.nx / 2 + 1) * g.ny + 127) / 128;
+        const int kc = predict_kchunk(g.nz, bx, 8 * sm_count());
+        k_predict2<<<dim3(bx, (g.nz + kc - 1) / kc), 128, 0, s>>>(g, b.F, b.u, b.v, b.w, b.us, b.vs, b.ws, kc);
     }
     if (g.csf && b.csf[0]) {  // surface tension (extension): normals, curvature, face accelerations
         const dim3 cb(32, 4, 2);
