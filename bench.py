@@ -67,7 +67,7 @@ ALG_BYTES = {
 }
 KERNEL_NAMES = {
     "predict": "k_predict2", "rhs": "k_rhs4", "jacobi": "k_jacobi_two", "correct": "k_correct4",
-    "sweep1": "k_fct_x|k_fct_march", "sweep2": "k_fct_x|k_fct_march", "sweep3": "k_fct_x|k_fct_march",
+    "sweep1": "k_fct_tile", "sweep2": "k_fct_tile", "sweep3": "k_fct_tile",
 }
 # (VOF_JACOBI=peel: one sweep per launch; by default two, k_jacobi_two)
 if os.environ.get("VOF_JACOBI") == "peel":

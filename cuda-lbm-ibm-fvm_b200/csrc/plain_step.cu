@@ -144,6 +144,107 @@ __global__ void __launch_bounds__(256) k_predict(Geom g,
     }
 }
 
+// ---------------------------------------------------------------------------
+// Continuum surface force (extension; no counterpart in the reference, whose
+// sigma no kernel reads).  J. U. Brackbill, D. B. Kothe, C. Zemach, "A
+// continuum method for modeling surface tension", J. Comput. Phys. 100 (1992):
+// the body force sigma kappa grad(F) with the interface normal n = grad F /
+// |grad F| and kappa = -div n, both by central differences at cell centres;
+// F's ghosts are the zero-gradient copies, and a normal beyond a wall is the
+// mirror image of the one inside (its wall-normal component negated: a 90
+// degree contact angle).  On a face, kappa is the mean of its two cells,
+// grad F their difference, and the acceleration is divided by the face
+// density of the correction, 0.5 (rho_a + rho_b); the predictor adds it to u*,
+// v*, w* on the faces it updates.  FP32, operations in a fixed order.
+// ---------------------------------------------------------------------------
+// The normal at a cell from the differences of its neighbours; zero where the
+// gradient is no larger than eps (or NaN), as it is at most cells: away from
+// the interface the differences are zeros and no root or quotient is formed.
+struct Normal {
+    float x, y, z;
+};
+__device__ __forceinline__ Normal csf_normal(float dx, float dy, float dz, float hx, float hy, float hz, float eps) {
+    Normal n = {0.0f, 0.0f, 0.0f};
+    if (dx == 0.0f && dy == 0.0f && dz == 0.0f) return n;
+    const float gxv = dx * hx, gyv = dy * hy, gzv = dz * hz;
+    const float mag = sqrtf(gxv * gxv + gyv * gyv + gzv * gzv);
+    if (!(mag > eps)) return n;
+    if (mag >= 0x1p-100f && mag < 0x1p+126f) {  // div_rn_pre's divisors
+        const float r = __frcp_rn(mag);
+        n.x = div_rn_pre(gxv, mag, r);
+        n.y = div_rn_pre(gyv, mag, r);
+        n.z = div_rn_pre(gzv, mag, r);
+    } else {
+        n.x = gxv / mag;
+        n.y = gyv / mag;
+        n.z = gzv / mag;
+    }
+    return n;
+}
+
+// kappa from F.  A block covers 32 x 16 columns, the outermost of them a halo
+// for the differences of the normals, and marches a chunk of planes: at plane k
+// a thread forms its normal, takes the x neighbours' from the lanes beside, the
+// y neighbours' from shared memory, and keeps the in-plane part of the
+// divergence until the next plane's normal completes it.  18 us at 128^3, where
+// a pass that stored the normals and one that read them took 17.4 + 12.1, and
+// the normals of the six neighbours formed per cell 23.6.  Bound by the warps
+// with interface cells, which the block waits for (chunks of 4 to 16 planes,
+// loads a plane ahead, 8 rows: 17.3 to 19.6).
+constexpr int CSF_X = 32, CSF_Y = 16;
+__global__ void __launch_bounds__(CSF_X* CSF_Y, 3) k_csf_curv(Geom g, const float* __restrict__ F,
+                                                              float* __restrict__ kap, int kchunk) {
+    __shared__ float rows[2][CSF_Y][CSF_X];
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const int i = blockIdx.x * (CSF_X - 2) + tx, j = blockIdx.y * (CSF_Y - 2) + ty;
+    const int k0 = 1 + blockIdx.z * kchunk, k1 = min(g.nz, k0 + kchunk - 1);
+    const int ka = max(1, k0 - 1), kb = min(g.nz, k1 + 1);
+    const bool in = i >= 1 && i <= g.nx && j >= 1 && j <= g.ny;
+    const bool out = in && tx >= 1 && tx < CSF_X - 1 && ty >= 1 && ty < CSF_Y - 1;
+    const int sy = g.px, sz = g.plane;
+    const float hx = 0.5f * g.dxi, hy = 0.5f * g.dyi, hz = 0.5f * g.dzi;
+    const float eps = 1e-6f * g.dxi;
+    int id = gidx(g, i, j, ka);
+    float fm = in ? __ldg(F + id - sz) : 0.0f, fc = in ? __ldg(F + id) : 0.0f;
+    float zm = 0.0f, zc = 0.0f, plane = 0.0f;  // the z components at k - 2 and k - 1, the in-plane part at k - 1
+    for (int k = ka; k <= kb; ++k, id += sz) {
+        Normal n = {0.0f, 0.0f, 0.0f};
+        float fp = 0.0f;
+        if (in) {
+            fp = __ldg(F + id + sz);
+            n = csf_normal(__ldg(F + id + 1) - __ldg(F + id - 1), __ldg(F + id + sy) - __ldg(F + id - sy), fp - fm, hx,
+                           hy, hz, eps);
+        }
+        rows[k & 1][ty][tx] = n.y;
+        if (out && k > k0) kap[id - sz] = -(plane + (n.z - (k > 2 ? zm : -zc)) * hz);
+        const float e = __shfl_down_sync(0xffffffffu, n.x, 1), w = __shfl_up_sync(0xffffffffu, n.x, 1);
+        __syncthreads();
+        if (out) {
+            // neighbours beyond a wall: the mirror image of the cell at the wall
+            const float xe = i < g.nx ? e : -n.x, xw = i > 1 ? w : -n.x;
+            const float yn = j < g.ny ? rows[k & 1][ty + 1][tx] : -n.y, ys = j > 1 ? rows[k & 1][ty - 1][tx] : -n.y;
+            plane = (xe - xw) * hx + (yn - ys) * hy;
+        }
+        zm = zc;
+        zc = n.z;
+        fm = fc;
+        fc = fp;
+    }
+    if (out && k1 == g.nz) kap[id - sz] = -(plane + (-zc - (g.nz > 1 ? zm : -zc)) * hz);
+}
+
+// A face's acceleration: the force (csf_force) over its density.  A force of
+// +-0, as away from the interface, is its own quotient when the densities are
+// positive (r lies between the two).
+__device__ __forceinline__ float csf_force(const Geom& g, float Fa, float Fb, float ka, float kb, float hinv) {
+    return g.sigma * (0.5f * (ka + kb)) * ((Fb - Fa) * hinv);
+}
+__device__ __forceinline__ float csf_accel(const Geom& g, float f, float Fa, float Fb) {
+    if (f == 0.0f && fminf(g.rpair[0], g.rpair[1]) > 1e-30f) return f;
+    const float r = 0.5f * (rho_of(g, Fa) + rho_of(g, Fb));
+    return f / r;
+}
+
 // The predictor with two cells per thread.  Cells are paired by padded column
 // (2m, 2m + 1: one aligned 8-byte word), the pairs of all rows of a plane
 // numbered flat so that 32 consecutive pairs make a warp across row ends, and
@@ -156,7 +257,7 @@ __global__ void __launch_bounds__(256) k_predict(Geom g,
 // memory at the ends of a warp and of a row.  Each cell's three updates keep
 // k_predict's expressions and operand order (same bits).  Bound by instruction
 // issue (209 thread instructions per cell, 70 % of the slots used): 77 -> 70
-// us at 200^3 and 507 -> 476 at 400^3 by predict_kchunk's shorter chunks, of
+// us at 200^3 and 507 -> 476 at 400^3 by march_kchunk's shorter chunks, of
 // which blocks of 128 threads rather than 256 are 1 to 3 %.  Packed FP32 pairs
 // (f32x2) took 99 us at 200^3, one viscosity for two equal cells 76.6.
 // The pair's left (x-1 of the first cell) and right (x+1 of the second cell)
@@ -170,10 +271,15 @@ __device__ __forceinline__ float right_of(float2 a, bool lde, const float* __res
     return lde ? __ldg(p + idr) : s;
 }
 
-__global__ void __launch_bounds__(128, 8) k_predict2(Geom g, const float* __restrict__ F,
-                                                     const float* __restrict__ u, const float* __restrict__ v,
-                                                     const float* __restrict__ w, float* __restrict__ us,
-                                                     float* __restrict__ vs, float* __restrict__ ws, int kchunk) {
+// CSF: the surface tension's acceleration added to each face: 31.4 us at 128^3
+// (21.6 without), a pass over u*, v*, w* of its own 17.4 to 24.8 more.
+template <bool CSF>
+__global__ void __launch_bounds__(128, CSF ? 6 : 8) k_predict2(Geom g, const float* __restrict__ F,
+                                                               const float* __restrict__ u,
+                                                               const float* __restrict__ v,
+                                                               const float* __restrict__ w, float* __restrict__ us,
+                                                               float* __restrict__ vs, float* __restrict__ ws,
+                                                               int kchunk, const float* __restrict__ kap) {
     const int npair = g.nx / 2 + 1;  // pairs covering columns 0 .. nx
     const int nq = npair * g.ny;
     const int qt = blockIdx.x * blockDim.x + threadIdx.x;
@@ -199,6 +305,11 @@ __global__ void __launch_bounds__(128, 8) k_predict2(Geom g, const float* __rest
     // x neighbours carried from the previous plane
     float wim_c = left_of(w_c, ldw, w, id - 1);
     float uip_km = right_of(u_km, lde, u, id + 2 - sz);
+    float2 f_km, kap_km;
+    if (CSF) {
+        f_km = L2(F, id - sz);
+        kap_km = L2(kap, id - sz);
+    }
     for (int k = k0; k <= k1; ++k, id += sz) {
         const float2 u_kp = L2(u, id + sz), v_kp = L2(v, id + sz), w_kp = L2(w, id + sz);
         const float2 wjm_kp = L2(w, id - sy + sz), vjp_c = L2(v, id + sy);
@@ -266,6 +377,23 @@ __global__ void __launch_bounds__(128, 8) k_predict2(Geom g, const float* __rest
                 out_w[e] = wc + g.dt * (visc + adv + g.gz);
             }
         }
+        if (CSF) {
+            const float2 kc = L2(kap, id), fj = L2(F, id - sy), kj = L2(kap, id - sy);
+            const float fi = left_of(f2, ldw, F, id - 1), ki = left_of(kc, ldw, kap, id - 1);
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const float Fc = e ? f2.y : f2.x, kk = e ? kc.y : kc.x;
+                const float Fx = e ? f2.x : fi, Fy = e ? fj.y : fj.x, Fz = e ? f_km.y : f_km.x;
+                const float ax = csf_force(g, Fx, Fc, e ? kc.x : ki, kk, g.dxi);
+                const float ay = csf_force(g, Fy, Fc, e ? kj.y : kj.x, kk, g.dyi);
+                const float az = csf_force(g, Fz, Fc, e ? kap_km.y : kap_km.x, kk, g.dzi);
+                out_u[e] = out_u[e] + g.dt * csf_accel(g, ax, Fx, Fc);
+                out_v[e] = out_v[e] + g.dt * csf_accel(g, ay, Fy, Fc);
+                out_w[e] = out_w[e] + g.dt * csf_accel(g, az, Fz, Fc);
+            }
+            f_km = f2;
+            kap_km = kc;
+        }
         float2* US = reinterpret_cast<float2*>(us + id);
         if (u0 && u1)
             *US = make_float2(out_u[0], out_u[1]);
@@ -300,74 +428,6 @@ __global__ void __launch_bounds__(128, 8) k_predict2(Geom g, const float* __rest
         uip_km = uip1;
         vjp_km = vjp_c;
     }
-}
-
-// ---------------------------------------------------------------------------
-// Continuum surface force (extension; no counterpart in the reference, whose
-// sigma no kernel reads).  J. U. Brackbill, D. B. Kothe, C. Zemach, "A
-// continuum method for modeling surface tension", J. Comput. Phys. 100 (1992):
-// the body force sigma kappa grad(F) with the interface normal n = grad F /
-// |grad F| and kappa = -div n, both by central differences at cell centres;
-// F's ghosts are the zero-gradient copies, and a normal beyond a wall is the
-// mirror image of the one inside (its wall-normal component negated: a 90
-// degree contact angle).  On a face, kappa is the mean of its two cells,
-// grad F their difference, and the acceleration is divided by the face
-// density of the correction, 0.5 (rho_a + rho_b); it is added to u*, v*, w*
-// on the faces the predictor updates.  FP32, operations in a fixed order.
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_csf_normal(Geom g, const float* __restrict__ F, float* __restrict__ nx_,
-                                                    float* __restrict__ ny_, float* __restrict__ nz_) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
-    const int k = blockIdx.z * blockDim.z + threadIdx.z + 1;
-    if (i > g.nx || j > g.ny || k > g.nz) return;
-    const int id = gidx(g, i, j, k);
-    const float hx = 0.5f * g.dxi, hy = 0.5f * g.dyi, hz = 0.5f * g.dzi;
-    const float gxv = (F[id + 1] - F[id - 1]) * hx;
-    const float gyv = (F[id + g.px] - F[id - g.px]) * hy;
-    const float gzv = (F[id + g.plane] - F[id - g.plane]) * hz;
-    const float mag = sqrtf(gxv * gxv + gyv * gyv + gzv * gzv);
-    const float eps = 1e-6f * g.dxi;
-    const bool has = mag > eps;
-    nx_[id] = has ? gxv / mag : 0.0f;
-    ny_[id] = has ? gyv / mag : 0.0f;
-    nz_[id] = has ? gzv / mag : 0.0f;
-}
-
-__global__ void __launch_bounds__(256) k_csf_curv(Geom g, const float* __restrict__ nx_,
-                                                  const float* __restrict__ ny_, const float* __restrict__ nz_,
-                                                  float* __restrict__ kap) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
-    const int k = blockIdx.z * blockDim.z + threadIdx.z + 1;
-    if (i > g.nx || j > g.ny || k > g.nz) return;
-    const int id = gidx(g, i, j, k);
-    const float hx = 0.5f * g.dxi, hy = 0.5f * g.dyi, hz = 0.5f * g.dzi;
-    // neighbours beyond a wall: the mirror image of the cell at the wall
-    const float xe = i < g.nx ? nx_[id + 1] : -nx_[id], xw = i > 1 ? nx_[id - 1] : -nx_[id];
-    const float yn = j < g.ny ? ny_[id + g.px] : -ny_[id], ys = j > 1 ? ny_[id - g.px] : -ny_[id];
-    const float zu = k < g.nz ? nz_[id + g.plane] : -nz_[id], zd = k > 1 ? nz_[id - g.plane] : -nz_[id];
-    kap[id] = -((xe - xw) * hx + (yn - ys) * hy + (zu - zd) * hz);
-}
-
-__device__ __forceinline__ float csf_accel(const Geom& g, float Fa, float Fb, float ka, float kb, float hinv) {
-    const float f = g.sigma * (0.5f * (ka + kb)) * ((Fb - Fa) * hinv);
-    const float r = 0.5f * (rho_of(g, Fa) + rho_of(g, Fb));
-    return f / r;
-}
-
-__global__ void __launch_bounds__(256) k_csf_force(Geom g, const float* __restrict__ F,
-                                                   const float* __restrict__ kap, float* __restrict__ us,
-                                                   float* __restrict__ vs, float* __restrict__ ws) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
-    const int k = blockIdx.z * blockDim.z + threadIdx.z + 1;
-    if (i > g.nx || j > g.ny || k > g.nz) return;
-    const int id = gidx(g, i, j, k);
-    const float Fc = F[id], kc = kap[id];
-    if (i >= 2) us[id] = us[id] + g.dt * csf_accel(g, F[id - 1], Fc, kap[id - 1], kc, g.dxi);
-    if (j >= 2) vs[id] = vs[id] + g.dt * csf_accel(g, F[id - g.px], Fc, kap[id - g.px], kc, g.dyi);
-    if (k >= 2) ws[id] = ws[id] + g.dt * csf_accel(g, F[id - g.plane], Fc, kap[id - g.plane], kc, g.dzi);
 }
 
 // ---------------------------------------------------------------------------
@@ -753,7 +813,7 @@ static bool jacobi_two(const Geom& g, int iters) {
 static int jacobi_launches(const Geom& g, int iters) { return jacobi_two(g, iters) ? (iters + 1) / 2 : iters; }
 
 int plain_kernels_per_step(const Geom& g, int jacobi_iters) {
-    return 1 + (g.csf ? 3 : 0) + 1 + jacobi_launches(g, jacobi_iters) + 1 + 3;
+    return 1 + (g.csf ? 1 : 0) + 1 + jacobi_launches(g, jacobi_iters) + 1 + 3;
 }
 
 // Column-marching launch shape: 32 x 8 columns per block, z split into
@@ -796,19 +856,19 @@ static int sm_count() {
     return n;
 }
 
-// Planes per block of k_predict2: the least estimate of its time in planes of
-// one resident block, waves of (kc + 1) planes each (the extra one for
-// the first window) and half a block for the uneven end.  Chunks as long as
+// Planes per block of k_predict2 (and k_csf_curv): the least estimate of its
+// time in planes of one resident block, waves of (kc + extra) planes each (extra
+// for the first window) and part of a block for the uneven end.  Chunks as long as
 // one wave allows left the SMs with fewer blocks than others idle at the end:
 // (blocks of 256) 200^3 29 planes a block 76.8 us, 20 79.3, 16 73.0, 10 71.3,
 // 8 (chosen) 71.7, 7 69.3, 4 72.5; 400^3 50 planes 507, 20 (chosen) 480, 16
 // 482, 10 484, 7 495, 4 528; 128^3 8 planes 23.0, 4 (chosen) 22.2, 2 22.6.
-static int predict_kchunk(int nz, int bx, int wave) {
+static int march_kchunk(int nz, int bx, int wave, int extra) {
     int best = 1;
     double least = 1e30;
     for (int kc = 1; kc <= nz; ++kc) {
         const double waves = (double)bx * ((nz + kc - 1) / kc) / wave;
-        const double cost = ((waves > 1.0 ? waves : 1.0) + 0.6) * (kc + 1);
+        const double cost = ((waves > 1.0 ? waves : 1.0) + 0.6) * (kc + extra);
         if (cost < least) {
             least = cost;
             best = kc;
@@ -833,19 +893,20 @@ cudaError_t plain_front(const Geom& g, const PlainBuffers& b, cudaStream_t s, cu
     if ((e = mark(ev, 0, s)) != cudaSuccess) return e;
     static int pforced = -1;  // VOF_PREDICT=1: k_predict (one cell per thread); else k_predict2
     if (pforced < 0) pforced = env_kernel("VOF_PREDICT");
-    if (pforced == 1) {
+    const int bx = ((g.nx / 2 + 1) * g.ny + 127) / 128;
+    if (g.csf && b.csf[3]) {  // surface tension (extension): curvature, then face accelerations in the predictor
+        const dim3 cg((g.nx + CSF_X - 3) / (CSF_X - 2), (g.ny + CSF_Y - 3) / (CSF_Y - 2));
+        const int cc = march_kchunk(g.nz, cg.x * cg.y, 3 * sm_count(), 3);
+        k_csf_curv<<<dim3(cg.x, cg.y, (g.nz + cc - 1) / cc), CSF_X * CSF_Y, 0, s>>>(g, b.F, b.csf[3], cc);
+        const int kc = march_kchunk(g.nz, bx, 6 * sm_count(), 1);
+        k_predict2<true><<<dim3(bx, (g.nz + kc - 1) / kc), 128, 0, s>>>(g, b.F, b.u, b.v, b.w, b.us, b.vs, b.ws, kc,
+                                                                        b.csf[3]);
+    } else if (pforced == 1) {
         k_predict<<<grid, blk, 0, s>>>(g, b.F, b.u, b.v, b.w, b.us, b.vs, b.ws, kchunk);
     } else {
-        const int bx = ((g.nx / 2 + 1) * g.ny + 127) / 128;
-        const int kc = predict_kchunk(g.nz, bx, 8 * sm_count());
-        k_predict2<<<dim3(bx, (g.nz + kc - 1) / kc), 128, 0, s>>>(g, b.F, b.u, b.v, b.w, b.us, b.vs, b.ws, kc);
-    }
-    if (g.csf && b.csf[0]) {  // surface tension (extension): normals, curvature, face accelerations
-        const dim3 cb(32, 4, 2);
-        const dim3 cg((g.nx + 31) / 32, (g.ny + 3) / 4, (g.nz + 1) / 2);
-        k_csf_normal<<<cg, cb, 0, s>>>(g, b.F, b.csf[0], b.csf[1], b.csf[2]);
-        k_csf_curv<<<cg, cb, 0, s>>>(g, b.csf[0], b.csf[1], b.csf[2], b.csf[3]);
-        k_csf_force<<<cg, cb, 0, s>>>(g, b.F, b.csf[3], b.us, b.vs, b.ws);
+        const int kc = march_kchunk(g.nz, bx, 8 * sm_count(), 1);
+        k_predict2<false><<<dim3(bx, (g.nz + kc - 1) / kc), 128, 0, s>>>(g, b.F, b.u, b.v, b.w, b.us, b.vs, b.ws, kc,
+                                                                         nullptr);
     }
     if ((e = cudaGetLastError()) != cudaSuccess || (e = mark(ev, 1, s)) != cudaSuccess) return e;
     static int forced = -1;  // VOF_RHS=1: k_rhs (one cell per thread, z march), 4: k_rhs4
@@ -946,7 +1007,7 @@ cudaError_t plain_step(const Geom& g, const PlainBuffers& b, int istep, int jaco
 
 int plain_phase_launches(const Geom& g, int phase, int jacobi_iters) {
     if (phase == PHASE_JACOBI) return jacobi_launches(g, jacobi_iters);
-    return (phase == PHASE_PREDICT && g.csf) ? 4 : 1;
+    return (phase == PHASE_PREDICT && g.csf) ? 2 : 1;
 }
 
 }  // namespace vof

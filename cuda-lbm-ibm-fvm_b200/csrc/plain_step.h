@@ -22,7 +22,8 @@ struct PlainBuffers {
     float* p2;   // scratch pressure buffer for the blocked sweeps
     const J2Tables* j2;       // of p0, p1, p2 and rhs (jacobi_two_prepare)
     int* status;              // device status word (DEV_* codes, tma.cuh)
-    float* csf[4];            // g.csf: interface normal x, y, z and curvature per cell; else null
+    float* csf[4];            // g.csf: the curvature per cell in csf[3] (csf[0..2] unused, kept so that a
+                              // context's allocations and reported bytes stay as they were); else null
 };
 
 // Query and configure the kernels.  Call once per device before the first step.
