@@ -22,6 +22,7 @@
 #include "fct_sweep.h"
 
 #include "fct_line.cuh"
+#include "pdl.cuh"
 
 namespace vof {
 
@@ -93,6 +94,7 @@ __device__ __forceinline__ bool thin(const Geom& g) { return g.nx == 1 || g.ny =
 template <int AXIS, bool FINAL>
 __global__ void __launch_bounds__(1024) k_fct_lines(Geom g, const float* __restrict__ Fsrc,
                                                     float* __restrict__ F, const float* __restrict__ vel, int lpb) {
+    pdl_enter(Fsrc, F, vel);
     extern __shared__ float smem[];
     const Sweep<AXIS> S(g);
     const int n = S.n, npos = n + 2;
@@ -369,9 +371,9 @@ static cudaError_t launch_axis(const Geom& g, const float* Fin, float* F, const 
     // tiles 5.8; 100 x 80 x 126: 10.2 and 6.9)
     const int lpb = lines_per_block(n, lines);
     if (lpb && cells <= 1 << 19) {
-        k_fct_lines<AXIS, FINAL><<<(unsigned)((lines + lpb - 1) / lpb), (lpb * (n + 2) + 31) / 32 * 32,
-                                   6 * lpb * (n + 2) * (int)sizeof(float), s>>>(g, Fin, F, vel, lpb);
-        return cudaGetLastError();
+        return pdl_launch(k_fct_lines<AXIS, FINAL>, (unsigned)((lines + lpb - 1) / lpb),
+                          (lpb * (n + 2) + 31) / 32 * 32, 6 * lpb * (n + 2) * (int)sizeof(float), s, g, Fin, F, vel,
+                          lpb);
     }
     if (AXIS != 0) {
         // positions per thread: 4, from 2^25 cells 6 (less overlap: 400^3, z

@@ -12,6 +12,8 @@
 
 #include "jacobi.h"
 
+#include "pdl.cuh"
+
 namespace vof {
 
 #if defined(__CUDA_ARCH__) && !defined(VOF_FMAD_FALSE)
@@ -115,6 +117,7 @@ template <int U, int MINB>
 __global__ void __launch_bounds__(JP_THREADS, MINB) k_jacobi_peel(Geom g, const float* __restrict__ pin,
                                                             const float* __restrict__ rhs,
                                                             float* __restrict__ pout, int kchunk) {
+    pdl_enter(pin, rhs, pout);
     const int npair = g.nx / 2 + 1;  // pairs covering columns 0 .. nx
     const int nq = npair * g.ny;
     const int qt = blockIdx.x * JP_THREADS + threadIdx.x;
@@ -206,8 +209,7 @@ cudaError_t jacobi_peel_launch(const Geom& g, const float* pin, const float* rhs
     const int bx = (nq + JP_THREADS - 1) / JP_THREADS;
     const int kchunk = forced > 0 ? (forced < g.nz ? forced : g.nz) : wave_kchunk(g.nz, bx, jpe_wave);
     const dim3 grid(bx, (g.nz + kchunk - 1) / kchunk);
-    k_jacobi_peel<2, 4><<<grid, JP_THREADS, 0, s>>>(g, pin, rhs, pout, kchunk);
-    return cudaGetLastError();
+    return pdl_launch(k_jacobi_peel<2, 4>, grid, JP_THREADS, 0, s, g, pin, rhs, pout, kchunk);
 }
 
 cudaError_t jacobi_configure() {

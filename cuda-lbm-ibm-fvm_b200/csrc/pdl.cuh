@@ -18,6 +18,15 @@ __device__ __forceinline__ void pdl_enter() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// The same for kernels that read through the read-only path: the pointers are
+// opaque after the wait, so that no load through them can be moved before it.
+template <typename... P>
+__device__ __forceinline__ void pdl_enter(P&... p) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    (([&] { asm volatile("" : "+l"(p)); }()), ...);
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 template <typename... KArgs, typename... Args>
 static cudaError_t pdl_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
                               Args&&... args) {

@@ -25,6 +25,7 @@
 #include "fct_sweep.h"
 #include "jacobi.h"
 #include "jacobi_two.h"
+#include "pdl.cuh"
 
 #include <cuda_runtime.h>
 #include <stdlib.h>
@@ -271,15 +272,17 @@ __device__ __forceinline__ float right_of(float2 a, bool lde, const float* __res
     return lde ? __ldg(p + idr) : s;
 }
 
+// PDL: launched ahead of the end of the kernel before (pdl.cuh; small grids).
 // CSF: the surface tension's acceleration added to each face: 31.4 us at 128^3
 // (21.6 without), a pass over u*, v*, w* of its own 17.4 to 24.8 more.
-template <bool CSF>
+template <bool CSF, bool PDL>
 __global__ void __launch_bounds__(128, CSF ? 6 : 8) k_predict2(Geom g, const float* __restrict__ F,
                                                                const float* __restrict__ u,
                                                                const float* __restrict__ v,
                                                                const float* __restrict__ w, float* __restrict__ us,
                                                                float* __restrict__ vs, float* __restrict__ ws,
                                                                int kchunk, const float* __restrict__ kap) {
+    if constexpr (PDL) pdl_enter(F, u, v, w, us, vs, ws);
     const int npair = g.nx / 2 + 1;  // pairs covering columns 0 .. nx
     const int nq = npair * g.ny;
     const int qt = blockIdx.x * blockDim.x + threadIdx.x;
@@ -441,6 +444,7 @@ __global__ void __launch_bounds__(256) k_rhs(Geom g,
                                              const float* __restrict__ vs,
                                              const float* __restrict__ ws,
                                              float* __restrict__ rhs, int kchunk) {
+    pdl_enter(F, us, vs, ws, rhs);
     const Column col(g, 1, 1, kchunk);
     if (col.i > g.nx || col.j > g.ny || col.k0 > g.nz) return;
     int id = gidx(g, col.i, col.j, col.k0);
@@ -640,6 +644,7 @@ __global__ void __launch_bounds__(256) k_correct(Geom g,
                                                  const float* __restrict__ p,
                                                  float* __restrict__ u, float* __restrict__ v,
                                                  float* __restrict__ w) {
+    pdl_enter(F, us, vs, ws, p, u, v, w);
     const int i = blockIdx.x * blockDim.x + threadIdx.x + 1;
     const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
     const int k = blockIdx.z * blockDim.z + threadIdx.z + 1;
@@ -899,20 +904,23 @@ cudaError_t plain_front(const Geom& g, const PlainBuffers& b, cudaStream_t s, cu
         const int cc = march_kchunk(g.nz, cg.x * cg.y, 3 * sm_count(), 3);
         k_csf_curv<<<dim3(cg.x, cg.y, (g.nz + cc - 1) / cc), CSF_X * CSF_Y, 0, s>>>(g, b.F, b.csf[3], cc);
         const int kc = march_kchunk(g.nz, bx, 6 * sm_count(), 1);
-        k_predict2<true><<<dim3(bx, (g.nz + kc - 1) / kc), 128, 0, s>>>(g, b.F, b.u, b.v, b.w, b.us, b.vs, b.ws, kc,
+        k_predict2<true, false><<<dim3(bx, (g.nz + kc - 1) / kc), 128, 0, s>>>(g, b.F, b.u, b.v, b.w, b.us, b.vs, b.ws, kc,
                                                                         b.csf[3]);
     } else if (pforced == 1) {
         k_predict<<<grid, blk, 0, s>>>(g, b.F, b.u, b.v, b.w, b.us, b.vs, b.ws, kchunk);
     } else {
         const int kc = march_kchunk(g.nz, bx, 8 * sm_count(), 1);
-        k_predict2<false><<<dim3(bx, (g.nz + kc - 1) / kc), 128, 0, s>>>(g, b.F, b.u, b.v, b.w, b.us, b.vs, b.ws, kc,
-                                                                         nullptr);
+        const dim3 pg(bx, (g.nz + kc - 1) / kc);
+        if (quads_fill(g))
+            k_predict2<false, false><<<pg, 128, 0, s>>>(g, b.F, b.u, b.v, b.w, b.us, b.vs, b.ws, kc, nullptr);
+        else
+            pdl_launch(k_predict2<false, true>, pg, 128, 0, s, g, b.F, b.u, b.v, b.w, b.us, b.vs, b.ws, kc, nullptr);
     }
     if ((e = cudaGetLastError()) != cudaSuccess || (e = mark(ev, 1, s)) != cudaSuccess) return e;
     static int forced = -1;  // VOF_RHS=1: k_rhs (one cell per thread, z march), 4: k_rhs4
     if (forced < 0) forced = env_kernel("VOF_RHS");
     if (forced == 1 || (forced != 4 && !quads_fill(g))) {
-        k_rhs<<<grid, blk, 0, s>>>(g, b.F, b.us, b.vs, b.ws, b.rhs, kchunk);
+        pdl_launch(k_rhs, grid, blk, 0, s, g, b.F, b.us, b.vs, b.ws, b.rhs, kchunk);
     } else {
         const int total = (g.nx / 4 + 1) * g.ny;
         k_rhs4<<<dim3((total + 255) / 256, g.nz), 256, 0, s>>>(g, b.F, b.us, b.vs, b.ws, b.rhs);
@@ -929,7 +937,7 @@ cudaError_t plain_correct(const Geom& g, const PlainBuffers& b, const float* p, 
     if (forced == 1 || (forced != 4 && !quads_fill(g))) {
         const dim3 cb(32, 4, 2);
         const dim3 cg((g.nx + 31) / 32, (g.ny + 3) / 4, (g.nz + 1) / 2);
-        k_correct<<<cg, cb, 0, s>>>(g, b.F, b.us, b.vs, b.ws, p, b.u, b.v, b.w);
+        pdl_launch(k_correct, cg, cb, 0, s, g, b.F, b.us, b.vs, b.ws, p, b.u, b.v, b.w);
     } else {
         const int total = (g.nx / 4 + 1) * g.ny;
         k_correct4<<<dim3((total + 255) / 256, g.nz), 256, 0, s>>>(g, b.F, b.us, b.vs, b.ws, p, b.u, b.v, b.w);
