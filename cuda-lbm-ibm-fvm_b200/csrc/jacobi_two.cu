@@ -67,12 +67,7 @@ __device__ __forceinline__ Quad quad(const float* a) {
 // Numerators below lo (ahead of a pressure front every block has some) take
 // div_rn_tiny's scaled quotient, in line; what that leaves (a possible
 // midpoint of the subnormal grid, huge or non-finite numerators) div_rn_pre.
-struct Range {
-    float lo, hi;
-    unsigned lo2;  // twice lo's bits, less one
-    bool tiny;     // div_rn_tiny's range holds for every |x| < lo
-};
-__device__ __forceinline__ Quad quotients(const Quad& x, const Quad& d, const Quad& rd, const Range& w) {
+__device__ __forceinline__ Quad quotients(const Quad& x, const Quad& d, const Quad& rd, const DivRange& w) {
     Quad q;
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
@@ -119,7 +114,7 @@ __device__ __forceinline__ Quad quotients(const Quad& x, const Quad& d, const Qu
 // products from above (up) and below (dn).
 __device__ __forceinline__ Quad update(const Quad& rhs, const Quad& X, float xw, float xe, float an, const Quad& n,
                                        float as, const Quad& s, const Quad& up, const Quad& dn, const Quad& d,
-                                       const Quad& rd, const Range& w) {
+                                       const Quad& rd, const DivRange& w) {
     Quad t;
 #pragma unroll
     for (int e = 0; e < 4; ++e)
@@ -183,18 +178,7 @@ __global__ void __launch_bounds__(J2_THREADS, 1) k_jacobi_two(Geom g, J2Plan P, 
             rd.v[e] = __frcp_rn(d.v[e]);
         }
     };
-    // div_rn_pre's fast quotients ask |x| >= 2^-100 and 2^-125 <= |q0| <= 2^96:
-    // with 2^-1 and 2^1 to spare for the rounding of q0 and of these bounds
-    Range w;
-    {
-        const float dmin = cx * (g.nx > 2) + cy * (g.ny > 2) + cz * (g.nz > 2);  // (a wall on each axis)
-        const float dmax = 2.0f * (cx + cy + cz);
-        w.lo = fmaxf(0x1p-100f, 0x1p-124f * dmax);
-        w.hi = fminf(0x1p+95f * dmin, 0x1p+126f);
-        w.lo2 = 2u * __float_as_uint(w.lo) - 1u;
-        // 2^-125 <= |x 2^64 / d| <= 2^96 and |x| < 2^-36 for 2^-149 <= |x| < lo
-        w.tiny = dmin >= 0x1p-30f && dmax <= 0x1p+38f && w.lo <= 0x1p-40f;
-    }
+    const DivRange w = div_range(g);
     Quad d, rd;
     diagonal(cz, cz, d, rd);
 

@@ -24,6 +24,7 @@
 
 #include "fct_sweep.h"
 #include "jacobi.h"
+#include "jacobi_cluster.h"
 #include "jacobi_two.h"
 #include "pdl.cuh"
 
@@ -761,8 +762,9 @@ __global__ void __launch_bounds__(256, 4) k_correct4(Geom g, const float* __rest
 // Host launchers
 // ---------------------------------------------------------------------------
 cudaError_t plain_configure() {
-    const cudaError_t e = jacobi_configure();
-    return e == cudaSuccess ? jacobi_two_configure() : e;
+    cudaError_t e = jacobi_configure();
+    if (e == cudaSuccess) e = jacobi_two_configure();
+    return e == cudaSuccess ? jacobi_cluster_configure() : e;
 }
 
 cudaError_t plain_density_pairs(Geom* g) {
@@ -800,22 +802,29 @@ bool plain_supported(const Geom& g) {
     return fct_supported(g.nx) && fct_supported(g.ny) && fct_supported(g.nz);
 }
 
-// Two sweeps per launch (k_jacobi_two), an odd count starting with one single
-// sweep (k_jacobi_peel), on grids of at least 2^19 cells; below, its march is
-// too short to pay for the halo (64^3: 30 steps 4.56 against 4.45 ms, 32^3
-// 1.65 against 1.59).  VOF_JACOBI=peel / two force either (same bits).
-static bool jacobi_two(const Geom& g, int iters) {
+// How the sweeps are launched.  All in one (k_jacobi_cluster) on grids of some
+// ten thousand cells; two per launch (k_jacobi_two), an odd count starting
+// with one single sweep (k_jacobi_peel), on grids of at least 2^19 cells;
+// between, one per launch: the march of two sweeps is too short there to pay
+// for its halo (64^3: 30 steps 4.56 against 4.45 ms, 32^3 1.65 against 1.59).
+// VOF_JACOBI=peel / two force either (same bits).
+enum class Sweeps { ONE, TWO, ALL };
+static Sweeps jacobi_kind(const Geom& g, int iters) {
     static int forced = -1;
     if (forced < 0) {
         const char* v = getenv("VOF_JACOBI");
-        forced = v && !strcmp(v, "peel") ? 1 : v && !strcmp(v, "two") ? 2 : 0;
+        forced = !v ? 0 : !strcmp(v, "peel") ? 1 : !strcmp(v, "two") ? 2 : 0;
     }
     // (a launch cannot end in the buffer it reads, where two sweeps have to end)
-    if (iters <= 2 || forced == 1) return false;
-    return forced == 2 || (long long)g.nx * g.ny * g.nz >= 1 << 19;
+    if (iters <= 2 || forced == 1) return Sweeps::ONE;
+    if (forced != 2 && jacobi_cluster_fits(g, iters)) return Sweeps::ALL;
+    return forced == 2 || (long long)g.nx * g.ny * g.nz >= 1 << 19 ? Sweeps::TWO : Sweeps::ONE;
 }
 
-static int jacobi_launches(const Geom& g, int iters) { return jacobi_two(g, iters) ? (iters + 1) / 2 : iters; }
+static int jacobi_launches(const Geom& g, int iters) {
+    const Sweeps q = jacobi_kind(g, iters);
+    return q == Sweeps::ALL ? 1 : q == Sweeps::TWO ? (iters + 1) / 2 : iters;
+}
 
 int plain_kernels_per_step(const Geom& g, int jacobi_iters) {
     return 1 + (g.csf ? 1 : 0) + 1 + jacobi_launches(g, jacobi_iters) + 1 + 3;
@@ -983,7 +992,10 @@ cudaError_t plain_pressure(const Geom& g, const PlainBuffers& b, int jacobi_iter
     float* pbuf[3] = {b.p0, b.p1, b.p2};
     const int src = *p_parity, dst = src ^ (jacobi_iters & 1);
     int cur = src;
-    if (jacobi_two(g, jacobi_iters)) {
+    const Sweeps kind = jacobi_kind(g, jacobi_iters);
+    if (kind == Sweeps::ALL) {
+        if ((e = jacobi_cluster_launch(g, pbuf, src, b.rhs, jacobi_iters, s)) != cudaSuccess) return e;
+    } else if (kind == Sweeps::TWO) {
         const int L = jacobi_launches(g, jacobi_iters);
         const bool detour = (L & 1) != (src != dst);
         for (int q = 0; q < L; ++q) {

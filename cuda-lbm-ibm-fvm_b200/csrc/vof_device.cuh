@@ -118,6 +118,30 @@ __device__ __forceinline__ float div_rn_pre(float x, float d, float rd) {
     return div_rn_tiny(x, d, rd);
 }
 
+// The numerators whose quotients by any diagonal of the pressure system
+// Markstein's correction rounds correctly, tested without the quotient: with
+// every |d| between the launch's least and greatest, lo <= |x| <= hi implies
+// div_rn_pre's conditions on x and q0.
+struct DivRange {
+    float lo, hi;
+    unsigned lo2;  // twice lo's bits, less one: 2 bits(x) - 1 >= lo2 for lo <= |x| and for 0
+    bool tiny;     // div_rn_tiny's range holds for every |x| < lo
+};
+__device__ __forceinline__ DivRange div_range(const Geom& g) {
+    DivRange w;
+    const float cx = g.dxi * g.dxi, cy = g.dyi * g.dyi, cz = g.dzi * g.dzi;
+    // div_rn_pre asks |x| >= 2^-100 and 2^-125 <= |q0| <= 2^96: with 2^-1 and
+    // 2^1 to spare for the rounding of q0 and of these bounds
+    const float dmin = cx * (g.nx > 2) + cy * (g.ny > 2) + cz * (g.nz > 2);  // (a wall on each axis)
+    const float dmax = 2.0f * (cx + cy + cz);
+    w.lo = fmaxf(0x1p-100f, 0x1p-124f * dmax);
+    w.hi = fminf(0x1p+95f * dmin, 0x1p+126f);
+    w.lo2 = 2u * __float_as_uint(w.lo) - 1u;
+    // 2^-125 <= |x 2^64 / d| <= 2^96 and |x| < 2^-36 for 2^-149 <= |x| < lo
+    w.tiny = dmin >= 0x1p-30f && dmax <= 0x1p+38f && w.lo <= 0x1p-40f;
+    return w;
+}
+
 // 1/x for a positive normal FP64 x, to within about one ulp (not always
 // correctly rounded), for the FP64 partial derivatives of the adjoint; the
 // FP32 forward never uses it.  Method: Newton-Raphson iteration for the
