@@ -39,6 +39,7 @@
 #include "fct_line.cuh"
 #include "fct_sweep.h"
 #include "jacobi_two.h"
+#include "pdl.cuh"
 
 namespace vof {
 
@@ -351,6 +352,7 @@ template <int DIR, int LPB>
 __global__ void __launch_bounds__(FA_THREADS) k_fct_adjoint(Geom g, const float* __restrict__ Fg,
                                                             const float* __restrict__ velg, double* __restrict__ lFg,
                                                             double* __restrict__ lvelg) {
+    pdl_enter(Fg, velg, lFg, lvelg);
     extern __shared__ __align__(16) unsigned char fa_smem[];
     const int n = slen<DIR>(g), N2 = n + 2, M = LPB * N2;
     double* sLX = reinterpret_cast<double*>(fa_smem);
@@ -940,6 +942,7 @@ __global__ void __launch_bounds__(FM_LANES * WARPS, DIR == 0 ? VOF_FM_MINB_X : V
 
 // ---- boundary copies, reversed ---------------------------------------------------
 __global__ void k_adj_bcF_z(Geom g, double* __restrict__ l) {
+    pdl_enter(l);
     const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
     if (i > g.nx + 1 || j > g.ny + 1) return;
     const int a = gidx(g, i, j, 0), b = gidx(g, i, j, 1), c = gidx(g, i, j, g.nz), d = gidx(g, i, j, g.nz + 1);
@@ -949,6 +952,7 @@ __global__ void k_adj_bcF_z(Geom g, double* __restrict__ l) {
     l[d] = 0.0;
 }
 __global__ void k_adj_bcF_x(Geom g, double* __restrict__ l) {
+    pdl_enter(l);
     const int j = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y * blockDim.y + threadIdx.y;
     if (j > g.ny + 1 || k > g.nz + 1) return;
     const int a = gidx(g, 0, j, k), b = gidx(g, 1, j, k), c = gidx(g, g.nx, j, k), d = gidx(g, g.nx + 1, j, k);
@@ -966,6 +970,7 @@ __global__ void k_adj_bcF_x(Geom g, double* __restrict__ l) {
     l[d] = 0.0;
 }
 __global__ void k_adj_bcF_y(Geom g, double* __restrict__ l) {
+    pdl_enter(l);
     const int i = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y * blockDim.y + threadIdx.y;
     if (i > g.nx + 1 || k > g.nz + 1) return;
     const int a = gidx(g, i, 0, k), b = gidx(g, i, 1, k), c = gidx(g, i, g.ny, k), d = gidx(g, i, g.ny + 1, k);
@@ -981,6 +986,7 @@ __device__ __forceinline__ void mv(double* l, int dst, int src) {
 }
 // set_bc_vel_k: u, v copied into the k ghosts, w zero at k = 1 and nz + 1.
 __global__ void k_adj_bcv_z(Geom g, double* __restrict__ lu, double* __restrict__ lv, double* __restrict__ lw) {
+    pdl_enter(lu, lv, lw);
     const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
     if (i > g.nx + 1 || j > g.ny + 1) return;
     const int k0 = gidx(g, i, j, 0), k1 = gidx(g, i, j, 1), kn = gidx(g, i, j, g.nz), kf = gidx(g, i, j, g.nz + 1);
@@ -994,6 +1000,7 @@ __global__ void k_adj_bcv_z(Geom g, double* __restrict__ lu, double* __restrict_
 // set_bc_vel_i: u zero at i = 1 and nx + 1, v, w copied into the i ghosts.
 // (Its rows are strided in memory: all loads are issued before the stores.)
 __global__ void k_adj_bcv_x(Geom g, double* __restrict__ lu, double* __restrict__ lv, double* __restrict__ lw) {
+    pdl_enter(lu, lv, lw);
     const int j = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y * blockDim.y + threadIdx.y;
     if (j > g.ny + 1 || k > g.nz + 1) return;
     const int i0 = gidx(g, 0, j, k), i1 = gidx(g, 1, j, k), in = gidx(g, g.nx, j, k), ir = gidx(g, g.nx + 1, j, k);
@@ -1021,6 +1028,7 @@ __global__ void k_adj_bcv_x(Geom g, double* __restrict__ lu, double* __restrict_
 }
 // set_bc_vel_j: v zero at j = 1 and ny + 1, u, w copied into the j ghosts.
 __global__ void k_adj_bcv_y(Geom g, double* __restrict__ lu, double* __restrict__ lv, double* __restrict__ lw) {
+    pdl_enter(lu, lv, lw);
     const int i = blockIdx.x * blockDim.x + threadIdx.x, k = blockIdx.y * blockDim.y + threadIdx.y;
     if (i > g.nx + 1 || k > g.nz + 1) return;
     const int j0 = gidx(g, i, 0, k), j1 = gidx(g, i, 1, k), jn = gidx(g, i, g.ny, k), jt = gidx(g, i, g.ny + 1, k);
@@ -1072,6 +1080,7 @@ __global__ void __launch_bounds__(256) k_adj_update(Geom g, Range R, const float
                                                     double* __restrict__ lp, double* __restrict__ lrho,
                                                     int pending, InvAp ia, double* __restrict__ mu_out,
                                                     double* __restrict__ lrhs) {
+    pdl_enter(F, p, lu, lv, lw, lp, lrho, mu_out, lrhs);
     RANGE_CELL(R);
     const int c = gidx(g, i, j, k);
     const int pos[3] = {i, j, k}, len[3] = {g.nx, g.ny, g.nz}, st[3] = {1, g.px, g.plane};
@@ -1120,6 +1129,7 @@ __global__ void __launch_bounds__(256) k_adj_update(Geom g, Range R, const float
 // mode 0: mu = lin / ap, lrhs = mu;  1: mu = -N lin / ap, lrhs += mu;  2: out = -N lin.
 __global__ void __launch_bounds__(256) k_adj_jacobi(Geom g, Range R, InvAp ia, const double* __restrict__ lin,
                                                     double* __restrict__ lout, double* __restrict__ lrhs, int mode) {
+    pdl_enter(lin, lout, lrhs);
     RANGE_CELL(R);
     const int c = gidx(g, i, j, k);
     if (mode == 2) {
@@ -1173,6 +1183,7 @@ template <int A, int B>
 __global__ void __launch_bounds__(AJ_T) k_adj_jacobi2(Geom g, InvAp ia, const double* __restrict__ lin,
                                                      double* __restrict__ lout, double* __restrict__ lrhs,
                                                      int kchunk) {
+    pdl_enter(lin, lout, lrhs);
     constexpr int WI = AJ_TX + 4, WA = AJ_TX + 2;
     __shared__ double sIn[3][AJ_NIN];
     __shared__ double sA[3][AJ_NA];
@@ -1473,7 +1484,7 @@ cudaError_t launch_fct_adjoint(const Geom& g, const float* Fs, const float* vel,
     if (DIR == 0) grid = dim3((g.ny + LPB - 1) / LPB, g.nz);
     else if (DIR == 1) grid = dim3((g.nx + LPB - 1) / LPB, g.nz);
     else grid = dim3((g.nx + LPB - 1) / LPB, g.ny);
-    k_fct_adjoint<DIR, LPB><<<grid, FA_THREADS, smem, s>>>(g, Fs, vel, lF, lvel);
+    pdl_launch(k_fct_adjoint<DIR, LPB>, grid, FA_THREADS, smem, s, g, Fs, vel, lF, lvel);
     return cudaGetLastError();
 }
 
@@ -1663,9 +1674,9 @@ cudaError_t reverse_step(AdjEngine& e, const StepData& d, int istep, cudaStream_
     // F boundary copies
     {
         const dim3 b(16, 16);
-        k_adj_bcF_z<<<dim3((g.nx + 2 + 15) / 16, (g.ny + 2 + 15) / 16), b, 0, s>>>(g, e.lF);
-        k_adj_bcF_x<<<dim3((g.ny + 2 + 15) / 16, (g.nz + 2 + 15) / 16), b, 0, s>>>(g, e.lF);
-        k_adj_bcF_y<<<dim3((g.nx + 2 + 15) / 16, (g.nz + 2 + 15) / 16), b, 0, s>>>(g, e.lF);
+        pdl_launch(k_adj_bcF_z, dim3((g.nx + 2 + 15) / 16, (g.ny + 2 + 15) / 16), b, 0, s, g, e.lF);
+        pdl_launch(k_adj_bcF_x, dim3((g.ny + 2 + 15) / 16, (g.nz + 2 + 15) / 16), b, 0, s, g, e.lF);
+        pdl_launch(k_adj_bcF_y, dim3((g.nx + 2 + 15) / 16, (g.nz + 2 + 15) / 16), b, 0, s, g, e.lF);
     }
     // the three sweeps, last first
     for (int q = 2; q >= 0; --q) {
@@ -1678,9 +1689,9 @@ cudaError_t reverse_step(AdjEngine& e, const StepData& d, int istep, cudaStream_
     // velocity boundary copies, then the correction
     {
         const dim3 b(16, 16);
-        k_adj_bcv_z<<<dim3((g.nx + 2 + 15) / 16, (g.ny + 2 + 15) / 16), b, 0, s>>>(g, e.lu, e.lv, e.lw);
-        k_adj_bcv_x<<<dim3((g.ny + 2 + 15) / 16, (g.nz + 2 + 15) / 16), b, 0, s>>>(g, e.lu, e.lv, e.lw);
-        k_adj_bcv_y<<<dim3((g.nx + 2 + 15) / 16, (g.nz + 2 + 15) / 16), b, 0, s>>>(g, e.lu, e.lv, e.lw);
+        pdl_launch(k_adj_bcv_z, dim3((g.nx + 2 + 15) / 16, (g.ny + 2 + 15) / 16), b, 0, s, g, e.lu, e.lv, e.lw);
+        pdl_launch(k_adj_bcv_x, dim3((g.ny + 2 + 15) / 16, (g.nz + 2 + 15) / 16), b, 0, s, g, e.lu, e.lv, e.lw);
+        pdl_launch(k_adj_bcv_y, dim3((g.nx + 2 + 15) / 16, (g.nz + 2 + 15) / 16), b, 0, s, g, e.lu, e.lv, e.lw);
     }
     const Range I = interior(g);
     const dim3 gi = grid_of(I);
@@ -1689,11 +1700,11 @@ cudaError_t reverse_step(AdjEngine& e, const StepData& d, int istep, cudaStream_
     // other lp buffer, lrhs = mu0)
     const bool fuse = !e.conv && e.jacobi_iters > 0;
     if (fuse) {
-        k_adj_update<true><<<gi, kBlk, 0, s>>>(g, I, d.F, d.p, e.lu, e.lv, e.lw, e.lp[e.lp_cur], e.lrho,
+        pdl_launch(k_adj_update<true>, gi, kBlk, 0, s, g, I, d.F, d.p, e.lu, e.lv, e.lw, e.lp[e.lp_cur], e.lrho,
                                                e.lp_pending ? 1 : 0, e.inv_ap, e.lp[e.lp_cur ^ 1], e.lrhs);
         e.lp_cur ^= 1;
     } else {
-        k_adj_update<false><<<gi, kBlk, 0, s>>>(g, I, d.F, d.p, e.lu, e.lv, e.lw, e.lp[e.lp_cur], e.lrho, 0,
+        pdl_launch(k_adj_update<false>, gi, kBlk, 0, s, g, I, d.F, d.p, e.lu, e.lv, e.lw, e.lp[e.lp_cur], e.lrho, 0,
                                                 e.inv_ap, nullptr, nullptr);
     }
     // lu, lv, lw now hold the adjoints of u*, v*, w*; the start velocity's
@@ -1723,9 +1734,9 @@ cudaError_t reverse_step(AdjEngine& e, const StepData& d, int istep, cudaStream_
             const double* in = e.lp[e.lp_cur];
             double* out = e.lp[e.lp_cur ^ 1];
             if (q + 1 < n1)
-                k_adj_jacobi2<1, 1><<<gj, bj, 0, s>>>(g, e.inv_ap, in, out, e.lrhs, kchunk);
+                pdl_launch(k_adj_jacobi2<1, 1>, gj, bj, 0, s, g, e.inv_ap, in, out, e.lrhs, kchunk);
             else
-                k_adj_jacobi<<<gi, kBlk, 0, s>>>(g, I, e.inv_ap, in, out, e.lrhs, 1);
+                pdl_launch(k_adj_jacobi, gi, kBlk, 0, s, g, I, e.inv_ap, in, out, e.lrhs, 1);
             e.lp_cur ^= 1;
         }
         e.lp_pending = true;
@@ -2212,7 +2223,7 @@ cudaError_t adj_backward(AdjEngine* e, const AdjState& fin, const double box[6],
     }
     if (e->lp_pending) {  // the first step's deferred last Jacobi stage: the initial pressure's adjoint
         const Range I = interior(g);
-        k_adj_jacobi<<<grid_of(I), kBlk, 0, s>>>(g, I, e->inv_ap, e->lp[e->lp_cur], e->lp[e->lp_cur ^ 1], e->lrhs, 2);
+        pdl_launch(k_adj_jacobi, grid_of(I), kBlk, 0, s, g, I, e->inv_ap, e->lp[e->lp_cur], e->lp[e->lp_cur ^ 1], e->lrhs, 2);
         e->lp_cur ^= 1;
         e->lp_pending = false;
     }
