@@ -15,10 +15,11 @@
 //   k_rhs4         the rhs expression of solve_p_jacobi_kernel voftrial1.cu:418-422
 //                  four cells per thread (k_rhs: one, marching z; VOF_RHS=1)
 //   k_jacobi_two   (jacobi_two.cu) two solve_p_jacobi_kernel sweeps per launch,  voftrial1.cu:401-439
-//                  four cells per thread (an odd one: k_jacobi_peel, jacobi.cu)
+//                  four cells per thread (an odd one: k_jacobi_peel, jacobi.cu);
+//                  all of them in one cluster on small grids: k_jacobi_cluster
 //   k_correct4     update_{u,v,w}_kernel + apply_bc_velocity   voftrial1.cu:441-493, 959-1051, 1107-1120
 //                  four cells per thread (k_correct: one; VOF_CORRECT=1)
-//   k_fct<AXIS,FINAL>  (fct_sweep.cu) fct_{x,y,z}_sweep_stage1..4, and on
+//   k_fct_tile     (fct_sweep.cu; k_fct_lines on small grids) fct_{x,y,z}_sweep_stage1..4, and on
 //                  the last sweep post_process_f_kernel + apply_bc_F   voftrial1.cu:502-905, 1053-1135
 #include "plain_step.h"
 
