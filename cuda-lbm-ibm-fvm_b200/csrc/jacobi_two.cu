@@ -36,8 +36,6 @@
 // slower.
 #include "jacobi_two.h"
 
-#include <math.h>
-
 #include <type_traits>
 
 #include "tma.cuh"
@@ -49,8 +47,6 @@ namespace vof {
 #endif
 
 namespace {
-
-constexpr int J2_THREADS = 512, J2_STAGES = 4, J2_SMEM = 220 * 1024;
 
 struct Quad {
     float v[4];
@@ -298,54 +294,6 @@ __global__ void __launch_bounds__(J2_THREADS, 1) k_jacobi_two(Geom g, J2Plan P, 
     }
 }
 
-static int j2_smem(int nq, int rows) {
-    const int plane = (((rows + 2) * 4 * nq * 4 + 127) & ~127);
-    return (2 * J2_STAGES + 2) * plane + J2_STAGES * (int)sizeof(uint64_t);
-}
-
-// The tiling with the least estimated time in units of microseconds: waves of
-// one block per SM, times the planes a block marches (its own, two of the halo
-// and about 1.5 to start), times a plane's cost (its warps' issue slots, not
-// below its latency).  At 200^3, 3 x 7 x 7 blocks of 19 x 31 quads and 29
-// planes; tilings of one, two, four or more columns of blocks or of other
-// lengths took 2 to 65 % longer there, two smaller blocks per SM 5 %.
-static J2Plan plan_of(const Geom& g) {
-    const int all = (g.nx + 1) / 4 + 1;  // quads covering columns 0 .. nx + 1
-    J2Plan best = {};
-    double least = 1e30;
-    for (int tx = 1; tx <= all; ++tx) {
-        J2Plan p;
-        p.tx = tx;
-        p.wq = (all + tx - 1) / tx;
-        p.hq = tx > 1 ? 1 : 0;
-        p.nq = p.wq + 2 * p.hq;
-        if ((tx - 1) * p.wq >= all) continue;  // an empty tile
-        if (p.nq > 64) continue;               // (a TMA box has at most 256 elements a side)
-        if (p.nq < 10 && tx > 1) break;
-        for (p.rows = g.ny < 12 ? 3 : 8; p.rows <= g.ny + 2 && p.rows * p.nq <= J2_THREADS; ++p.rows) {
-            p.smem = j2_smem(p.nq, p.rows);
-            if (p.smem > J2_SMEM) break;
-            p.ty = (g.ny + p.rows - 3) / (p.rows - 2);
-            p.threads = (p.nq * p.rows + 31) / 32 * 32;
-            const double plane = fmax(0.45, 0.15 + 0.04 * (p.threads / 32));
-            const int tiles = p.tx * p.ty;
-            for (int waves = (tiles + 147) / 148, last = waves + 12; waves <= last; ++waves) {
-                int nch = waves * 148 / tiles;
-                if (nch > g.nz) nch = g.nz;
-                p.kc = (g.nz + nch - 1) / nch;
-                const int blocks = tiles * ((g.nz + p.kc - 1) / p.kc);
-                const double cost = (double)((blocks + 147) / 148) * (p.kc + 3.5) * plane;
-                if (cost < least) {
-                    least = cost;
-                    best = p;
-                }
-                if (p.kc <= 8 || nch == g.nz) break;
-            }
-        }
-    }
-    return best;
-}
-
 // Columns [from, px) of every row set to 1 (a warp per row; px - from <= 31).
 __global__ void __launch_bounds__(256) k_fill_padding(float* a, int px, int from, int rows) {
     const int i = from + (threadIdx.x & 31);
@@ -354,7 +302,7 @@ __global__ void __launch_bounds__(256) k_fill_padding(float* a, int px, int from
 }
 
 cudaError_t jacobi_two_prepare(const Geom& g, float* const field[4], J2Tables* t, cudaStream_t s) {
-    t->plan = plan_of(g);
+    t->plan = j2_plan(g.nx, g.ny, g.nz);
     const J2Plan& p = t->plan;
     for (int q = 0; q < 4; ++q) {
         const cudaError_t e =

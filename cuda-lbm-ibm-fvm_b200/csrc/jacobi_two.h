@@ -3,18 +3,10 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include "jacobi_two_plan.h"
 #include "vof_device.cuh"
 
 namespace vof {
-
-// Tiling of one launch: blocks of nq x rows quads (four cells of a row) march
-// kc planes; the outermost hq quads (where tiles neighbour along x) and the
-// first and last row are halo.
-struct J2Plan {
-    int nq, rows, hq, wq;  // quads per row of the tile, rows, halo quads a side, quads a tile writes
-    int tx, ty, kc;        // tiles along x and y, planes per block
-    int threads, smem;
-};
 
 // What the launches on one set of buffers need, made once: the tiling and the
 // TMA descriptors of the three pressure buffers and of the right-hand side.
