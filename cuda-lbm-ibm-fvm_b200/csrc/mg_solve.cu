@@ -16,7 +16,8 @@
 // 126 (10 V-cycles) 0.16 where it was 3.1 ms; 24^3 0.09 where it was 0.6-0.8.
 // Smaller grids keep one multigrid V-cycle per correction: programs there
 // read the cycle count and meet its cap (solver_stats, max_outer), which a
-// direct solve would always leave at 1.  Its vectors:
+// direct solve would always leave at 1; so do boxes so flat that a column's
+// alpha would round to 1/2 (sp_takes).  Its vectors:
 //   MIXED: every multigrid vector stored in BF16, arithmetic in FP32;
 //   FP64:  the same cycle with FP64 storage and arithmetic (the yardstick).
 // VOF_MG_PAIRS (0 or 1: row or paired kernels) in the environment keeps the
@@ -1129,7 +1130,7 @@ cudaError_t mg_create(const Geom& g, int mode, MgSolver* m, cudaStream_t s, size
     m->pairs = 1;
     if (const char* v = getenv("VOF_MG_PAIRS")) m->pairs = atoi(v) != 0;
     m->nlev = mg_plan(g, m->lv, MG_MAX_LEVELS);
-    m->direct = m->lv[0].ncell >= MG_DIRECT_CELLS && !getenv("VOF_MG_PAIRS");
+    m->direct = m->lv[0].ncell >= MG_DIRECT_CELLS && sp_takes(g.nx, g.ny, g.dxi, g.dyi, g.dzi) && !getenv("VOF_MG_PAIRS");
     if (m->direct) m->nlev = 1;
     cudaError_t e;
     const size_t vb = m->direct ? sizeof(double) : mode == MG_MIXED ? sizeof(__nv_bfloat16) : sizeof(double);

@@ -25,7 +25,7 @@
 // one step ahead).  The last transform (along x) adds into the pressure.
 //
 // Columns (k_zcr).  With the column's equation scaled to
-//   e_k - alpha (e_{k-1} + e_{k+1}) = q_k,   0 < alpha < 1/2,
+//   e_k - alpha (e_{k-1} + e_{k+1}) = q_k,   0 < alpha < 1/2 (in FP64 too: sp_takes),
 // and the zero-gradient ends mirrored (an even sequence of period 2 nz), one
 // step of cyclic reduction (R. W. Hockney, J. ACM 12(1), 1965) applied to
 // every row keeps that form with stride 2 s,
@@ -33,7 +33,7 @@
 // up to the factor 1 / (1 - 2 alpha^2), which is collected and applied at
 // the end.  alpha falls quadratically: the loop ends when it is below 2^-60
 // in every column of the block, after some 5 steps for most columns and 13
-// for the slowest at nz = 200.  All terms of a step have the sign of their
+// for the slowest at nz = 200 (SP_ZCR_STEPS at most).  All terms of a step have the sign of their
 // q's weights (no cancellation).  At 200^3 it takes 76 us; two more dense
 // transforms and the division took 225.  The constant column's system is singular:
 // one warp sums it twice and removes the mean.
@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(ZCR_THREADS, 2) k_zcr(int nx, int ny, int nz, 
         __syncthreads();
     }
     int s = 1;  // stride modulo the period 2 nz
-    while (__syncthreads_or(al > 0x1p-60)) {
+    for (int step = 0; step < SP_ZCR_STEPS && __syncthreads_or(al > 0x1p-60); ++step) {
 #pragma unroll 4
         for (int k = row; k < nz; k += ROWS) {
             int a = k - s, b = k + s;  // mirrored into 0 .. nz-1: the sequence is even about -1/2 with period 2 nz

@@ -7,6 +7,7 @@
 
 #include <new>
 
+#include "spectral_plan.h"
 #include "vof_device.cuh"
 
 namespace vof {

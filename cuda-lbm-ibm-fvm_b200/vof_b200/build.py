@@ -45,7 +45,7 @@ SOURCES = {
     "host_pull.cu": [],
     "apply_bc.cu": [],
 }
-HEADERS = ["vof_device.cuh", "tma.cuh", "plain_step.h", "fct_sweep.h", "fct_line.cuh", "jacobi.h", "jacobi_two.h", "jacobi_two_plan.h", "jacobi_cluster.h", "host_pull.h", "mg_solve.h", "spectral.h", "pdl.cuh",
+HEADERS = ["vof_device.cuh", "tma.cuh", "plain_step.h", "fct_sweep.h", "fct_line.cuh", "jacobi.h", "jacobi_two.h", "jacobi_two_plan.h", "jacobi_cluster.h", "host_pull.h", "mg_solve.h", "spectral.h", "spectral_plan.h", "pdl.cuh",
            "reduce.h", "adjoint.h", "apply_bc.h"]
 
 
