@@ -231,7 +231,7 @@ __device__ __forceinline__ int block_linear() { return blockIdx.x + gridDim.x * 
 
 __global__ void __launch_bounds__(MG_THREADS) k_fold2(const double* __restrict__ partial, int nblk,
                                                       double* __restrict__ out, double* host_out) {
-    pdl_enter();
+    pdl_enter(partial, out, host_out);
     double a = 0, b = 0;
     for (int q = threadIdx.x; q < nblk; q += blockDim.x) {
         a += partial[2 * q];
@@ -262,7 +262,7 @@ __global__ void __launch_bounds__(MG_THREADS) k_mg_smooth(MgLevel L, const S* __
                                                           S* __restrict__ eout, const S* __restrict__ b,
                                                           const double* __restrict__ bsum, double alpha, double beta,
                                                           int read_prev) {
-    pdl_enter();
+    pdl_enter(ein, eout, b, bsum);
     using C = typename St<S>::C;
     LEVEL_TILE(L);
     if (!active) return;
@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(MG_THREADS) k_mg_smooth2(MgLevel L, const __nv
                                                            __nv_bfloat16* __restrict__ eout,
                                                            const __nv_bfloat16* __restrict__ b, double alpha_d,
                                                            double beta_d, int read_prev) {
-    pdl_enter();
+    pdl_enter(ein, eout, b);
     const int pi = blockIdx.x * MG_BX + threadIdx.x;  // pair index along x
     const int i0 = 2 * pi;
     const int j = blockIdx.y * MG_BY + threadIdx.y;
@@ -447,7 +447,7 @@ __global__ void __launch_bounds__(MG_FLAT_THREADS) k_mg_smooth_pairs(MgLevel L, 
                                                                      unsigned* __restrict__ eout,
                                                                      const unsigned* __restrict__ b, float alpha,
                                                                      float beta) {
-    pdl_enter();
+    pdl_enter(ein, eout, b);
     using namespace pk;
     const int npr = L.nx >> 1, npl = npr * L.ny;
     const int q0 = blockIdx.x * MG_FLAT_THREADS + threadIdx.x;
@@ -495,7 +495,7 @@ __global__ void __launch_bounds__(MG_FLAT_THREADS) k_mg_restrict_pairs(MgLevel F
                                                                        const unsigned* __restrict__ b, MgLevel Cl,
                                                                        __nv_bfloat16* __restrict__ bc,
                                                                        __nv_bfloat16* __restrict__ ec) {
-    pdl_enter();
+    pdl_enter(e, b, bc, ec);
     using namespace pk;
     const int cn = Cl.nx * Cl.ny;
     const int q0 = blockIdx.x * MG_FLAT_THREADS + threadIdx.x;
@@ -556,7 +556,7 @@ __global__ void __launch_bounds__(MG_FLAT_THREADS) k_mg_restrict_pairs(MgLevel F
 __global__ void __launch_bounds__(MG_FLAT_THREADS) k_mg_prolong_pairs(MgLevel F, unsigned* __restrict__ e,
                                                                       MgLevel Cl,
                                                                       const __nv_bfloat16* __restrict__ ecrs) {
-    pdl_enter();
+    pdl_enter(e, ecrs);
     using namespace pk;
     const int cn = Cl.nx * Cl.ny;
     const int q0 = blockIdx.x * MG_FLAT_THREADS + threadIdx.x;
@@ -612,7 +612,7 @@ template <typename S>
 __global__ void __launch_bounds__(MG_THREADS) k_mg_restrict(MgLevel F, const S* __restrict__ e,
                                                             const S* __restrict__ b, MgLevel Cl,
                                                             S* __restrict__ bc, S* __restrict__ ec) {
-    pdl_enter();
+    pdl_enter(e, b, bc, ec);
     using T = St<S>;
     using C = typename T::C;
     LEVEL_TILE(Cl);
@@ -639,7 +639,7 @@ template <typename S>
 __global__ void __launch_bounds__(RW_THREADS) k_mg_restrict_wide(MgLevel F, const S* __restrict__ e,
                                                                  const S* __restrict__ b, MgLevel Cl,
                                                                  S* __restrict__ bc, S* __restrict__ ec) {
-    pdl_enter();
+    pdl_enter(e, b, bc, ec);
     using T = St<S>;
     using C = typename T::C;
     __shared__ C part[RW_THREADS / 32];
@@ -668,7 +668,7 @@ __global__ void __launch_bounds__(RW_THREADS) k_mg_restrict_wide(MgLevel F, cons
 template <typename S>
 __global__ void __launch_bounds__(MG_THREADS) k_mg_prolong(MgLevel F, S* __restrict__ e, MgLevel Cl,
                                                            const S* __restrict__ ec) {
-    pdl_enter();
+    pdl_enter(e, ec);
     LEVEL_TILE(F);
     if (!active) return;
     for (int k = k0; k < k1; ++k) prolong_cell<S>(F, e, Cl, ec, i, j, k);
@@ -677,7 +677,7 @@ __global__ void __launch_bounds__(MG_THREADS) k_mg_prolong(MgLevel F, S* __restr
 template <typename S>
 __global__ void __launch_bounds__(MG_THREADS) k_level_sum(MgLevel L, const S* __restrict__ b,
                                                           double* __restrict__ partial) {
-    pdl_enter();
+    pdl_enter(b, partial);
     LEVEL_TILE(L);
     double a = 0, z = 0;
     if (active)
@@ -693,7 +693,7 @@ __global__ void __launch_bounds__(MG_THREADS) k_level_sum(MgLevel L, const S* __
 template <typename R>
 __global__ void __launch_bounds__(MG_THREADS) k_sum_rhs(Geom g, MgLevel L0, const R* __restrict__ rhs,
                                                         double* __restrict__ partial) {
-    pdl_enter();
+    pdl_enter(rhs, partial);
     LEVEL_TILE(L0);
     double a = 0, z = 0;
     if (active)
@@ -712,7 +712,7 @@ __global__ void __launch_bounds__(MG_THREADS) k_resid0(Geom g, MgLevel L0, const
                                                        const double* __restrict__ sums, const double* __restrict__ p,
                                                        S* __restrict__ b0, S* __restrict__ e0,
                                                        double* __restrict__ partial) {
-    pdl_enter();
+    pdl_enter(rhs, sums, p, b0, e0, partial);
     using T = St<S>;
     using C = typename T::C;
     LEVEL_TILE(L0);
@@ -758,7 +758,7 @@ __global__ void __launch_bounds__(MG_THREADS) k_smooth_update(Geom g, MgLevel L0
                                                               const S* __restrict__ prev, const S* __restrict__ b,
                                                               double* __restrict__ p, double alpha, double beta,
                                                               int read_prev) {
-    pdl_enter();
+    pdl_enter(ein, prev, b, p);
     using T = St<S>;
     using C = typename T::C;
     LEVEL_TILE(L0);
@@ -783,7 +783,7 @@ __global__ void __launch_bounds__(MG_THREADS) k_smooth_update(Geom g, MgLevel L0
 template <typename S>
 __global__ void __launch_bounds__(MG_THREADS) k_update64(Geom g, MgLevel L0, double* __restrict__ p,
                                                          const S* __restrict__ e) {
-    pdl_enter();
+    pdl_enter(p, e);
     LEVEL_TILE(L0);
     if (!active) return;
     for (int k = k0; k < k1; ++k) p[gidx(g, i + 1, j + 1, k + 1)] += (double)St<S>::ld(e, (k * L0.ny + j) * L0.nx + i);
@@ -791,7 +791,7 @@ __global__ void __launch_bounds__(MG_THREADS) k_update64(Geom g, MgLevel L0, dou
 
 __global__ void __launch_bounds__(MG_THREADS) k_sum_p(Geom g, MgLevel L0, const double* __restrict__ p,
                                                       double* __restrict__ partial) {
-    pdl_enter();
+    pdl_enter(p, partial);
     LEVEL_TILE(L0);
     double a = 0, z = 0;
     if (active)
@@ -806,7 +806,7 @@ __global__ void __launch_bounds__(MG_THREADS) k_sum_p(Geom g, MgLevel L0, const 
 // p -= mean(p) (gauge), p32 = float(p) on the interior.
 __global__ void __launch_bounds__(MG_THREADS) k_gauge_cast(Geom g, MgLevel L0, double* __restrict__ p,
                                                            const double* __restrict__ sump, float* __restrict__ p32) {
-    pdl_enter();
+    pdl_enter(p, sump, p32);
     LEVEL_TILE(L0);
     if (!active) return;
     const double mean = sump[0] / (double)L0.ncell;
@@ -820,7 +820,7 @@ __global__ void __launch_bounds__(MG_THREADS) k_gauge_cast(Geom g, MgLevel L0, d
 
 __global__ void __launch_bounds__(MG_THREADS) k_widen(Geom g, MgLevel L0, const float* __restrict__ p32,
                                                       double* __restrict__ p) {
-    pdl_enter();
+    pdl_enter(p32, p);
     LEVEL_TILE(L0);
     if (!active) return;
     for (int k = k0; k < k1; ++k) {
@@ -1530,12 +1530,12 @@ struct DCell {
 template <typename R>
 __global__ void __launch_bounds__(D_THREADS) k_dsum(Geom g, int kchunk, const R* __restrict__ rhs, double* partial,
                                                     unsigned* ticket, double* out) {
-    pdl_enter();
+    pdl_enter(rhs, partial, ticket, out);
     const DCell t(g, kchunk);
     double a = 0.0;
     int id = t.id;
 #pragma unroll 8
-    for (int k = t.k0; k <= t.k1; ++k, id += g.plane) a += (double)rhs[id];
+    for (int k = t.k0; k <= t.k1; ++k, id += g.plane) a += (double)__ldg(rhs + id);
     fold3(a, 0.0, 0.0, partial, ticket, out, nullptr);
 }
 
@@ -1548,18 +1548,18 @@ __global__ void __launch_bounds__(D_THREADS, 4) k_dresid(Geom g, int kchunk, dou
                                                          const double* __restrict__ p, double* __restrict__ r0,
                                                          double* partial, unsigned* ticket, double* out,
                                                          double* host_out) {
-    pdl_enter();
+    pdl_enter(rhs, sums, p, r0, partial, ticket, out, host_out);
     const DCell t(g, kchunk);
     double rr = 0.0, bb = 0.0, pp = 0.0;
-    const double mean = sums[0] / ((double)g.nx * g.ny * g.nz);
+    const double mean = __ldg(sums) / ((double)g.nx * g.ny * g.nz);
     // a wall's neighbour is the cell itself (its difference is 0)
     const int ow = t.i > 0 ? -1 : 0, oe = t.i < g.nx - 1 ? 1 : 0;
     const int os = t.j > 0 ? -g.px : 0, on = t.j < g.ny - 1 ? g.px : 0;
     int id = t.id, c0 = ((t.k0 - 1) * g.ny + t.j) * g.nx + t.i;
     double pm = 0.0, pc = 0.0;
     if (t.k1 > 0) {
-        pc = p[id];
-        pm = t.k0 > 1 ? p[id - g.plane] : pc;
+        pc = __ldg(p + id);
+        pm = t.k0 > 1 ? __ldg(p + id - g.plane) : pc;
     }
     for (int k = t.k0; k <= t.k1; k += DK, id += DK * g.plane, c0 += DK * g.nx * g.ny) {
         double c[DK + 1], w[DK], e[DK], s[DK], n[DK], b[DK];
@@ -1567,12 +1567,12 @@ __global__ void __launch_bounds__(D_THREADS, 4) k_dresid(Geom g, int kchunk, dou
 #pragma unroll
         for (int q = 0; q < DK; ++q) {
             const int at = id + (k + q <= t.k1 ? q : 0) * g.plane;
-            c[q + 1] = p[k + q < g.nz ? at + g.plane : at];
-            w[q] = p[at + ow];
-            e[q] = p[at + oe];
-            s[q] = p[at + os];
-            n[q] = p[at + on];
-            b[q] = (double)rhs[at];
+            c[q + 1] = __ldg(p + (k + q < g.nz ? at + g.plane : at));
+            w[q] = __ldg(p + at + ow);
+            e[q] = __ldg(p + at + oe);
+            s[q] = __ldg(p + at + os);
+            n[q] = __ldg(p + at + on);
+            b[q] = (double)__ldg(rhs + at);
         }
 #pragma unroll
         for (int q = 0; q < DK; ++q) {
@@ -1599,7 +1599,7 @@ __global__ void __launch_bounds__(D_THREADS, 4) k_dresid(Geom g, int kchunk, dou
 // p -= mean(p) (gauge), p32 = float(p) on the interior.
 __global__ void __launch_bounds__(D_THREADS) k_dgauge(Geom g, int kchunk, const double* __restrict__ sum,
                                                       double* __restrict__ p, float* __restrict__ p32) {
-    pdl_enter();
+    pdl_enter(sum, p, p32);
     const DCell t(g, kchunk);
     const double mean = sum[0] / ((double)g.nx * g.ny * g.nz);
     int id = t.id;

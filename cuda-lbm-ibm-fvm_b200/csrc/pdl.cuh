@@ -18,15 +18,24 @@ __device__ __forceinline__ void pdl_enter() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-// The same for kernels that read through the read-only path: the pointers are
-// opaque after the wait, so that no load through them can be moved before it.
-// The step's small-grid kernels, the layout copies and the adjoint's short
-// kernels begin so (24 x 20 x 16, one step a call: 640 -> 485 us for six); the
-// large grids' kernels do not: registers for the opaque pointers cost them 1 %.
+// The same for kernels that read through __restrict__ pointers or __ldg: such a
+// load may be moved before the wait, whose memory clobber does not bind it.
+// The pointers are opaque after the wait, and known to be global (as opaque
+// generic ones they cost the V-cycle 2 to 3 %: 16^3 MIXED 663 -> 683 us a step;
+// so 668, and the reverse pass of 64^3 x 40 steps takes 6.84 ms for 7.04).
+// The solve's kernels, the step's small-grid ones, the layout copies and the
+// adjoint's short kernels begin so (24 x 20 x 16, one step a call: 640 -> 485
+// us for six); the large grids' kernels do not: registers for the opaque
+// pointers cost them 1 %.
 template <typename... P>
 __device__ __forceinline__ void pdl_enter(P&... p) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    (([&] { asm volatile("" : "+l"(p)); }()), ...);
+    (([&] {
+         size_t a = __cvta_generic_to_global(p);
+         asm volatile("" : "+l"(a));
+         p = static_cast<P>(__cvta_global_to_generic(a));
+     }()),
+     ...);
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 

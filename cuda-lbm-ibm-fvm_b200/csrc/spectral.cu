@@ -107,7 +107,7 @@ __device__ __forceinline__ void gemm(const double* __restrict__ f, int m, int kt
 
 // AXIS 0 (x) or 1 (y); BACK: the transform back (along x: added into p).
 template <int AXIS, bool BACK, int TN, bool WIDE>
-__global__ void __launch_bounds__(WIDE ? 512 : 256, WIDE ? 1 : 3) k_dct(SpArgs A, double* __restrict__ w) {
+__global__ void __launch_bounds__(WIDE ? 512 : 256, WIDE ? 1 : 3) k_dct(SpArgs A, double* w) {
     pdl_enter();
     if (reached(A.stop)) return;
     constexpr int NT = TN / 8, P = TN + 4;  // P = 4 (mod 16): a B fragment's words are on distinct banks
@@ -213,8 +213,8 @@ __global__ void __launch_bounds__(WIDE ? 512 : 256, WIDE ? 1 : 3) k_dct(SpArgs A
 constexpr int ZCR_THREADS = 512;
 
 template <int TN>
-__global__ void __launch_bounds__(ZCR_THREADS, 2) k_zcr(int nx, int ny, int nz, double az, const double* __restrict__ lx,
-                                             const double* __restrict__ ly, double* __restrict__ w, SpStop stop) {
+__global__ void __launch_bounds__(ZCR_THREADS, 2) k_zcr(int nx, int ny, int nz, double az, const double* lx,
+                                             const double* ly, double* w, SpStop stop) {
     pdl_enter();
     if (reached(stop)) return;
     extern __shared__ __align__(16) double Z[];
