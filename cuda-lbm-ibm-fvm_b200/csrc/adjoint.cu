@@ -1835,8 +1835,7 @@ cudaError_t adj_create(const Geom& g, int jacobi_iters, int mg_mode, double tol,
         const float ap = -(ae + aw + an + as + af + ab);
         e->inv_ap.v[f] = ap != 0.0f ? 1.0 / (double)ap : 0.0;
     }
-    float* const mapped[4] = {e->wb.p0, e->wb.p1, e->wb.p2, e->wb.rhs};
-    if ((r = jacobi_two_prepare(g, mapped, &e->j2, s)) != cudaSuccess) return r;
+    if ((r = plain_prepare(g, jacobi_iters, &e->wb, &e->j2, s)) != cudaSuccess) return r;
     if (e->conv) {
         if ((r = alloc((void**)&e->p64, db)) != cudaSuccess) return r;
         if ((r = mg_create(g, mg_mode, &e->mg_fwd, s, &e->bytes)) != cudaSuccess) return r;
@@ -1846,7 +1845,6 @@ cudaError_t adj_create(const Geom& g, int jacobi_iters, int mg_mode, double tol,
             return r;
         }
     }
-    e->wb.j2 = &e->j2;
     e->wb.status = e->status;
     return cudaStreamSynchronize(s);
 }

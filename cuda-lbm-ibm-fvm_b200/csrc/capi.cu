@@ -387,16 +387,12 @@ int vof_create(const vof_params* p, void* stream, vof_ctx** out) {
     c->b.vs = c->fields[VOF_FIELD_VSTAR - 1];
     c->b.ws = c->fields[VOF_FIELD_WSTAR - 1];
     c->b.rhs = c->fields[VOF_FIELD_RHS - 1];
-    c->b.j2 = &c->j2;
     c->b.status = c->d_status;
     c->p_parity = 0;
-    {
-        float* const mapped[4] = {c->b.p0, c->b.p1, c->b.p2, c->b.rhs};
-        if ((e = vof::jacobi_two_prepare(c->g, mapped, &c->j2, c->stream)) != cudaSuccess) {
-            c->last_cuda_error = (int)e;
-            free_ctx(c);
-            return VOF_E_UNSUPPORTED;
-        }
+    if ((e = vof::plain_prepare(c->g, p->jacobi_iters, &c->b, &c->j2, c->stream)) != cudaSuccess) {
+        c->last_cuda_error = (int)e;
+        free_ctx(c);
+        return VOF_E_UNSUPPORTED;
     }
 
     if ((e = vof::plain_configure()) != cudaSuccess || (e = vof::plain_density_pairs(&c->g)) != cudaSuccess ||

@@ -8,6 +8,16 @@ namespace vof {
 constexpr int J2_THREADS = 512, J2_STAGES = 4, J2_SMEM = 220 * 1024;
 constexpr int J2_BOX = 256;  // most elements a side of a TMA box may have
 
+// Whether `iters` sweeps of a grid run two per launch where nothing else takes
+// them (forced: 1 one per launch, 2 two, 0 by size).  From 2^19 cells: below,
+// the march of two sweeps is too short to pay for its halo (64^3: 30 steps 4.56
+// against 4.45 ms, 32^3 1.65 against 1.59; from 128^3 up two are faster).  A
+// launch cannot end in the buffer it reads, where two sweeps have to end.
+inline bool j2_chosen(int nx, int ny, int nz, int iters, int forced) {
+    if (iters <= 2 || forced == 1) return false;
+    return forced == 2 || (long long)nx * ny * nz >= 1 << 19;
+}
+
 // Tiling of one launch: blocks of nq x rows quads (four cells of a row) march
 // kc planes; the outermost hq quads (where tiles neighbour along x) and the
 // first and last row are halo.

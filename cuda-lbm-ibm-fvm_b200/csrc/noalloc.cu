@@ -126,10 +126,6 @@ extern "C" int vof_step_noalloc(const vof_params* prm, float* F, float* u, float
     if (e == cudaSuccess) e = vof::plain_density_pairs_on(&g, tail, s);
     if (e != cudaSuccess) return VOF_E_CUDA;
 
-    vof::J2Tables j2;
-    float* const mapped[4] = {f[8], f[9], f[10], f[7]};
-    if (vof::jacobi_two_prepare(g, mapped, &j2, s) != cudaSuccess) return VOF_E_UNSUPPORTED;
-
     vof::PlainBuffers b;
     memset(&b, 0, sizeof(b));
     b.F = f[0];
@@ -143,8 +139,9 @@ extern "C" int vof_step_noalloc(const vof_params* prm, float* F, float* u, float
     b.p0 = f[8];
     b.p1 = f[9];
     b.p2 = f[10];
-    b.j2 = &j2;
     b.status = status;
+    vof::J2Tables j2;
+    if (vof::plain_prepare(g, prm->jacobi_iters, &b, &j2, s) != cudaSuccess) return VOF_E_UNSUPPORTED;
     int parity = 0;
     e = vof::plain_step(g, b, istep, prm->jacobi_iters, &parity, s, nullptr);
     // The status word first: on a timed-out wait the step's results are

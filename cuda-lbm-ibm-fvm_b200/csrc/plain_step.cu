@@ -805,21 +805,30 @@ bool plain_supported(const Geom& g) {
 
 // How the sweeps are launched.  All in one (k_jacobi_cluster) on grids of some
 // ten thousand cells; two per launch (k_jacobi_two), an odd count starting
-// with one single sweep (k_jacobi_peel), on grids of at least 2^19 cells;
-// between, one per launch: the march of two sweeps is too short there to pay
-// for its halo (64^3: 30 steps 4.56 against 4.45 ms, 32^3 1.65 against 1.59).
-// VOF_JACOBI=peel / two force either (same bits).
+// with one single sweep (k_jacobi_peel), on large ones (j2_chosen); between,
+// one per launch.  VOF_JACOBI=peel / two force either (same bits).
 enum class Sweeps { ONE, TWO, ALL };
-static Sweeps jacobi_kind(const Geom& g, int iters) {
+static int jacobi_forced() {
     static int forced = -1;
     if (forced < 0) {
         const char* v = getenv("VOF_JACOBI");
         forced = !v ? 0 : !strcmp(v, "peel") ? 1 : !strcmp(v, "two") ? 2 : 0;
     }
-    // (a launch cannot end in the buffer it reads, where two sweeps have to end)
+    return forced;
+}
+static Sweeps jacobi_kind(const Geom& g, int iters) {
+    const int forced = jacobi_forced();
     if (iters <= 2 || forced == 1) return Sweeps::ONE;
     if (forced != 2 && jacobi_cluster_fits(g, iters)) return Sweeps::ALL;
-    return forced == 2 || (long long)g.nx * g.ny * g.nz >= 1 << 19 ? Sweeps::TWO : Sweeps::ONE;
+    return j2_chosen(g.nx, g.ny, g.nz, iters, forced) ? Sweeps::TWO : Sweeps::ONE;
+}
+
+cudaError_t plain_prepare(const Geom& g, int jacobi_iters, PlainBuffers* b, J2Tables* t, cudaStream_t s) {
+    b->j2 = nullptr;
+    if (!j2_chosen(g.nx, g.ny, g.nz, jacobi_iters, jacobi_forced())) return cudaSuccess;
+    float* const field[4] = {b->p0, b->p1, b->p2, b->rhs};
+    b->j2 = t;
+    return jacobi_two_prepare(g, field, t, s);
 }
 
 static int jacobi_launches(const Geom& g, int iters) {
@@ -997,6 +1006,7 @@ cudaError_t plain_pressure(const Geom& g, const PlainBuffers& b, int jacobi_iter
     if (kind == Sweeps::ALL) {
         if ((e = jacobi_cluster_launch(g, pbuf, src, b.rhs, jacobi_iters, s)) != cudaSuccess) return e;
     } else if (kind == Sweeps::TWO) {
+        if (!b.j2) return cudaErrorInvalidValue;
         const int L = jacobi_launches(g, jacobi_iters);
         const bool detour = (L & 1) != (src != dst);
         for (int q = 0; q < L; ++q) {

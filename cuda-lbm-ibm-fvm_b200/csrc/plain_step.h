@@ -20,7 +20,7 @@ struct PlainBuffers {
     float* p0;   // Jacobi ping-pong pair (DeviceFields::p / ::pt)
     float* p1;
     float* p2;   // scratch pressure buffer for the blocked sweeps
-    const J2Tables* j2;       // of p0, p1, p2 and rhs (jacobi_two_prepare)
+    const J2Tables* j2;       // of p0, p1, p2 and rhs where two sweeps a launch run (plain_prepare), else null
     int* status;              // device status word (DEV_* codes, tma.cuh)
     float* csf[4];            // g.csf: the curvature per cell in csf[3] (csf[0..2] unused, kept so that a
                               // context's allocations and reported bytes stay as they were); else null
@@ -28,6 +28,11 @@ struct PlainBuffers {
 
 // Query and configure the kernels.  Call once per device before the first step.
 cudaError_t plain_configure();
+
+// Fill t for b's pressure buffers and right-hand side and set b->j2, where
+// `jacobi_iters` sweeps of this grid run two per launch; b->j2 is null
+// elsewhere.  Once per set of buffers, before the first step on them.
+cudaError_t plain_prepare(const Geom& g, int jacobi_iters, PlainBuffers* b, J2Tables* t, cudaStream_t s);
 
 // Fill g->rpair / g->qpair (the density pairs of pure cells and dt over
 // them) with device arithmetic.  Call once per context.

@@ -24,3 +24,7 @@ extern "C" int check_plans(const int* from, const int* to, const int* step, int*
             }
     return broken;
 }
+
+extern "C" int chosen(int nx, int ny, int nz, int iters, int forced) {
+    return vof::j2_chosen(nx, ny, nz, iters, forced);
+}

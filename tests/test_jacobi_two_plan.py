@@ -36,6 +36,18 @@ def test_tilings_stay_within_the_limits_of_a_launch(plans, first, last, step):
     assert broken == 0, (broken, tuple(bad))
 
 
+@pytest.mark.parametrize("shape,iters,forced,want", [((24, 20, 16), 10, 0, 0), ((64, 64, 64), 10, 0, 0),
+                                                     ((80, 80, 80), 10, 0, 0), ((81, 81, 81), 10, 0, 1),
+                                                     ((128, 64, 64), 10, 0, 1), ((905, 905, 905), 10, 0, 1),
+                                                     ((200, 200, 200), 2, 0, 0), ((200, 200, 200), 3, 0, 1),
+                                                     ((200, 200, 200), 10, 1, 0), ((6, 5, 4), 10, 2, 1),
+                                                     ((6, 5, 4), 2, 2, 0), ((200, 200, 200), 0, 2, 0)])
+def test_tables_are_made_where_two_sweeps_run(plans, shape, iters, forced, want):
+    """Only these calls set up the two-sweep launch: a step of a small grid in
+    caller's memory does so on every call, for nothing otherwise."""
+    assert plans.chosen(*shape, iters, forced) == want
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("shape", [(1, 512, 512), (2, 256, 256), (3, 253, 905), (1, 800, 800), (2, 700, 400)])
 def test_two_dimensional_grids_bitwise_vs_oracle(cuda, V, orc, shape):
