@@ -56,6 +56,13 @@ __device__ __forceinline__ Quad quad(const float* a) {
     return {{t.x, t.y, t.z, t.w}};
 }
 
+// The greatest of three, NaN if one is.
+__device__ __forceinline__ float max_nan(float a, float b, float c) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
 // Quotients x / d of a quad by Markstein's correction (div_rn_pre).  Its range
 // test on the numerators alone: with every |d| between the launch's least and
 // greatest, lo <= |x| <= hi implies div_rn_pre's conditions on x and q0.  One
@@ -63,7 +70,11 @@ __device__ __forceinline__ Quad quad(const float* a) {
 // Numerators below lo (ahead of a pressure front every block has some) take
 // div_rn_tiny's scaled quotient, in line; what that leaves (a possible
 // midpoint of the subnormal grid, huge or non-finite numerators) div_rn_pre.
-__device__ __forceinline__ Quad quotients(const Quad& x, const Quad& d, const Quad& rd, const DivRange& w) {
+// Every quotient that is not finite comes that way, and rest_of(q) sees it
+// (a maximum that keeps NaN: a fmaxf would drop it).
+template <typename Rest>
+__device__ __forceinline__ Quad quotients(const Quad& x, const Quad& d, const Quad& rd, const DivRange& w,
+                                          Rest&& rest_of) {
     Quad q;
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
@@ -75,7 +86,7 @@ __device__ __forceinline__ Quad quotients(const Quad& x, const Quad& d, const Qu
 #pragma unroll
     for (int e = 0; e < 4; ++e) m[e] = 2u * __float_as_uint(x.v[e]) - 1u;
     const unsigned least = min(min(m[0], m[1]), min(m[2], m[3]));
-    const float most = fmaxf(fmaxf(fabsf(x.v[0]), fabsf(x.v[1])), fmaxf(fabsf(x.v[2]), fabsf(x.v[3])));
+    const float most = max_nan(max_nan(fabsf(x.v[0]), fabsf(x.v[1]), fabsf(x.v[2])), fabsf(x.v[3]), 0.0f);
     if (!(least >= w.lo2 && most <= w.hi)) {
         bool rest = !(w.tiny && most <= w.hi);
 #pragma unroll
@@ -100,6 +111,7 @@ __device__ __forceinline__ Quad quotients(const Quad& x, const Quad& d, const Qu
                 if (e == 2) q.v[2] = y;
                 if (e == 3) q.v[3] = y;
             }
+            rest_of(q);
         }
     }
     return q;
@@ -108,15 +120,16 @@ __device__ __forceinline__ Quad quotients(const Quad& x, const Quad& d, const Qu
 // The updates of a quad: right-hand sides, x products of the quad and of the
 // cells beside it, y neighbours (north, south) with their coefficients, z
 // products from above (up) and below (dn).
+template <typename Rest>
 __device__ __forceinline__ Quad update(const Quad& rhs, const Quad& X, float xw, float xe, float an, const Quad& n,
                                        float as, const Quad& s, const Quad& up, const Quad& dn, const Quad& d,
-                                       const Quad& rd, const DivRange& w) {
+                                       const Quad& rd, const DivRange& w, Rest&& rest_of) {
     Quad t;
 #pragma unroll
     for (int e = 0; e < 4; ++e)
         t.v[e] = rhs.v[e] - (e < 3 ? X.v[e + 1] : xe) - (e > 0 ? X.v[e - 1] : xw) - an * n.v[e] - as * s.v[e] -
                  up.v[e] - dn.v[e];
-    return quotients(t, d, rd, w);
+    return quotients(t, d, rd, w, rest_of);
 }
 
 __device__ __forceinline__ Quad scaled(float c, const Quad& a) { return {{c * a.v[0], c * a.v[1], c * a.v[2], c * a.v[3]}}; }
@@ -183,6 +196,15 @@ __global__ void __launch_bounds__(J2_THREADS, 1) k_jacobi_two(Geom g, J2Plan P, 
     const bool first = own && j >= 1 && j <= g.ny && i0 >= 0 && i0 <= g.nx;
     const bool out = first && r >= 1 && r <= rows - 2 && q >= P.hq && q < nq - P.hq;
     const bool whole = i0 >= 1 && i0 + 3 <= g.nx;
+    // The first sweep forms values for a row's ghosts as well, which enter the
+    // second through a coefficient of 0 only: not where they overflow (huge
+    // values in the ghosts of p, any in those of rhs).
+    auto clear = [&](Quad& q) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            if (i0 + e < 1 || i0 + e > g.nx) q.v[e] = 0.0f;
+    };
+    auto leave = [](Quad&) {};
     const int so = (r + 1) * pitch + 4 * q;  // own quad in a plane slot (row 0: the row before the tile)
 
     Quad zm, zc, pc;  // A: cz * p(k-1), cz * p(k), p(k)
@@ -221,9 +243,9 @@ __global__ void __launch_bounds__(J2_THREADS, 1) k_jacobi_two(Geom g, J2Plan P, 
                 if (EDGE) {
                     Quad dk, rdk;
                     diagonal(k < g.nz ? cz : 0.0f, k > 1 ? cz : 0.0f, dk, rdk);
-                    in = update(rk, X, xw, xe, an, quad(pk + pitch), as, quad(pk - pitch), up, zm, dk, rdk, w);
+                    in = update(rk, X, xw, xe, an, quad(pk + pitch), as, quad(pk - pitch), up, zm, dk, rdk, w, clear);
                 } else {
-                    in = update(rk, X, xw, xe, an, quad(pk + pitch), as, quad(pk - pitch), up, zm, d, rd, w);
+                    in = update(rk, X, xw, xe, an, quad(pk + pitch), as, quad(pk - pitch), up, zm, d, rd, w, clear);
                 }
             }
             zm = zc;
@@ -241,9 +263,9 @@ __global__ void __launch_bounds__(J2_THREADS, 1) k_jacobi_two(Geom g, J2Plan P, 
                 if (EDGE) {
                     Quad dk, rdk;
                     diagonal(k <= g.nz ? cz : 0.0f, k > 2 ? cz : 0.0f, dk, rdk);
-                    v = update(rp, X, xw, xe, an, quad(sb + pitch), as, quad(sb - pitch), wn, wm, dk, rdk, w);
+                    v = update(rp, X, xw, xe, an, quad(sb + pitch), as, quad(sb - pitch), wn, wm, dk, rdk, w, leave);
                 } else {
-                    v = update(rp, X, xw, xe, an, quad(sb + pitch), as, quad(sb - pitch), wn, wm, d, rd, w);
+                    v = update(rp, X, xw, xe, an, quad(sb + pitch), as, quad(sb - pitch), wn, wm, d, rd, w, leave);
                 }
                 if (whole) {
                     *reinterpret_cast<float4*>(o) = make_float4(v.v[0], v.v[1], v.v[2], v.v[3]);

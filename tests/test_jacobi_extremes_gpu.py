@@ -1,5 +1,7 @@
-"""The three Jacobi kernels (one sweep per launch, two, all in a cluster) with
-quotients beyond the fast division's range, bit for bit against the FP32 oracle.
+"""The three Jacobi kernels (one sweep per launch, two, all in a cluster) at the
+ends of the FP32 range, bit for bit against the FP32 oracle: quotients beyond
+the fast division's range in the cells, and ghost cells whose values enter only
+through zero coefficients but would overflow in any arithmetic of their own.
 The choice by size is forced (VOF_JACOBI is read once per process: in a child;
 without it these grids take the cluster)."""
 import os
@@ -25,6 +27,8 @@ for q in range(int(sys.argv[3])):
     nx, ny, nz, iters = (int(x) for x in f["case"])
     with V.Solver(V.default_params(nx, ny, nz, dt=2e-4, gy=0.0, gz=-9.81, jacobi_iters=iters)) as s:
         s.upload_state(**{k: f[k] for k in "Fuvwp"})
+        if "rhs" in f:
+            s.upload("rhs", f["rhs"])
         s.step(1)
         np.savez(f"{sys.argv[2]}/out{q}.npz", **s.state())
 """
@@ -61,3 +65,23 @@ def test_quotients_beyond_the_fast_division(cuda, V, orc, tmp_path, env):
         assert np.isfinite(want["p"]).all() and np.abs(want["p"]).max() > 1e24
         for k in ("p", "u", "v", "w", "F"):  # (NaN where the correction of such pressures has one)
             assert np.array_equal(got[k], want[k], equal_nan=True), (prm.shape, k)
+
+
+@KERNELS
+def test_ghosts_that_would_overflow(cuda, V, orc, tmp_path, env):
+    cases = []
+    for shape in SHAPES:
+        prm = params(V, *shape)
+        state = ic.random_state(prm, seed=sum(shape), vel_scale=0.5)
+        rng = np.random.default_rng(sum(shape))
+        ghost = np.ones(prm.shape, dtype=bool)
+        ghost[1:-1, 1:-1, 1:-1] = False
+        state["p"][ghost] = (rng.choice([-1.0, 1.0], prm.shape) * 10.0 ** rng.uniform(30, 38, prm.shape))[ghost]
+        rhs = np.zeros(prm.shape, dtype=np.float32)
+        rhs[ghost] = rng.choice([np.nan, np.inf, -np.inf], prm.shape)[ghost]
+        cases.append((prm, dict(state, rhs=rhs)))
+    for (prm, fields), got in zip(cases, step(tmp_path, env, cases)):
+        want = orc.run_f32(prm, {k: fields[k] for k in "Fuvwp"}, 1, 1)
+        assert np.isfinite(want["p"][1:-1, 1:-1, 1:-1]).all()
+        for k in ("p", "u", "v", "w", "F"):
+            assert np.array_equal(got[k], want[k]), (prm.shape, k, int((got[k] != want[k]).sum()))
