@@ -10,7 +10,6 @@
 #include <string.h>
 
 #include <atomic>
-#include <system_error>
 #include <thread>
 
 namespace vof {
@@ -91,8 +90,8 @@ cudaError_t host_pull(HostPull* h, void* dst, const void* src, size_t bytes, cud
     int started = 1;
     try {
         for (; started < PULL_THREADS; ++started) th[started] = std::thread(work, started);
-    } catch (const std::system_error&) {
-        // (no more threads: their slices below)
+    } catch (...) {
+        // (no thread to be had, or no memory for its state: their slices below)
     }
     work(0);
     for (int t = started; t < PULL_THREADS; ++t) work(t);
