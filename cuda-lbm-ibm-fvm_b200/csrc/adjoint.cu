@@ -1835,7 +1835,7 @@ cudaError_t adj_create(const Geom& g, int jacobi_iters, int mg_mode, double tol,
         const float ap = -(ae + aw + an + as + af + ab);
         e->inv_ap.v[f] = ap != 0.0f ? 1.0 / (double)ap : 0.0;
     }
-    if ((r = plain_prepare(g, jacobi_iters, &e->wb, &e->j2, s)) != cudaSuccess) return r;
+    if ((r = plain_prepare(g, e->conv ? 0 : jacobi_iters, &e->wb, &e->j2, s)) != cudaSuccess) return r;
     if (e->conv) {
         if ((r = alloc((void**)&e->p64, db)) != cudaSuccess) return r;
         if ((r = mg_create(g, mg_mode, &e->mg_fwd, s, &e->bytes)) != cudaSuccess) return r;

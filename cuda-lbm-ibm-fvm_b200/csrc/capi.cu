@@ -389,7 +389,7 @@ int vof_create(const vof_params* p, void* stream, vof_ctx** out) {
     c->b.rhs = c->fields[VOF_FIELD_RHS - 1];
     c->b.status = c->d_status;
     c->p_parity = 0;
-    if ((e = vof::plain_prepare(c->g, p->jacobi_iters, &c->b, &c->j2, c->stream)) != cudaSuccess) {
+    if ((e = vof::plain_prepare(c->g, c->conv ? 0 : p->jacobi_iters, &c->b, &c->j2, c->stream)) != cudaSuccess) {
         c->last_cuda_error = (int)e;
         free_ctx(c);
         return VOF_E_UNSUPPORTED;

@@ -22,9 +22,11 @@
 // ahead, from one thread, and fill with zeros outside the field.  The first
 // sweep's values on the tile's edge (one row, one quad) are computed twice.
 //
-// What bounds it: instruction issue, at 33 thread instructions per cell and
-// sweep on the tile and 45 with its halo (the one-sweep kernel k_jacobi_peel:
-// 55) and two thirds of the issue slots used while a block runs; DRAM and L2
+// What bounds it: instruction issue and its barrier, at 33 thread instructions
+// per cell and sweep on the tile and 41 with its halo (the one-sweep kernel
+// k_jacobi_peel: 55), with half of the issue slots used while a block runs (15
+// warps an SM; stalls on the barrier, shared memory, fixed latency and the
+// scheduler's choice about alike; at 200^3 39 us a launch).  DRAM and L2
 // see one read of p and rhs and one write of p per two sweeps.  Without any
 // load it takes 5 % less, so the copies are hidden.  Measured on a B200, whole
 // passes of steps against one sweep per launch: 400^3 in flow 16.6 -> 15.1 ms

@@ -18,7 +18,12 @@ constexpr double MG_RATIO_FINE = 6.0;   // eigenvalue ratio they damp (the 2x-co
 constexpr int MG_NU_COARSE = 8;         // pre/post degree on the small levels
 constexpr double MG_RATIO_COARSE = 30.0;  // wider: these levels may coarsen by 3, 5 or 7
 constexpr int MG_MAX_NU = 8;
-// Grids of at least this many cells are solved directly (spectral.cu).
+// Grids of at least this many cells are solved directly (spectral.cu).  Not the
+// crossover of the two, which lies below 8^3 (us a step on a B200, direct
+// against V-cycles in MIXED / FP64: 8^3 68, 257 / 221; 12^3 74, 445 / 311; 16^3
+// 75, 668 / 458; 20^3 81, 409 / 316; 24^3 82, 555 / 402): smaller grids keep the
+// V-cycle because programs there read its count and meet its cap (solver_stats,
+// max_outer), which a direct solve leaves at 1.
 constexpr int MG_DIRECT_CELLS = 8192;
 constexpr int MG_COARSE_SWEEPS = 100;   // sweeps on a coarsest level too large for the dense solve
 constexpr int MG_MAX_LEVELS = 16;

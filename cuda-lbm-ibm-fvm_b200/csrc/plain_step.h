@@ -31,7 +31,7 @@ cudaError_t plain_configure();
 
 // Fill t for b's pressure buffers and right-hand side and set b->j2, where
 // `jacobi_iters` sweeps of this grid run two per launch; b->j2 is null
-// elsewhere.  Once per set of buffers, before the first step on them.
+// elsewhere (the convergent modes run none: 0).  Once per set of buffers, before the first step on them.
 cudaError_t plain_prepare(const Geom& g, int jacobi_iters, PlainBuffers* b, J2Tables* t, cudaStream_t s);
 
 // Fill g->rpair / g->qpair (the density pairs of pure cells and dt over

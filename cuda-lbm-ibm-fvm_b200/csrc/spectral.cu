@@ -18,7 +18,7 @@
 // asynchronously (all of them in flight at once: by registers, 8 loads a
 // thread, a 200^3 pass took 15 us longer), folded there, each warp forms 16
 // rows of both parts for all TN lines, and the results go back in place.  At
-// 200^3 a pass takes 85 to 105 us with the tensor pipe 50 to 60 % busy (its
+// 200^3 a pass takes 85 to 105 us with the tensor pipe 62 to 68 % busy (its
 // floor is 51 us: 1.86 GFLOP with the padding of 100 rows to 112 x 104); the
 // rest is the blocks' load and store phases, which three blocks an SM overlap
 // in part.  The matrices come in fragment order straight from L2 (coalesced,
