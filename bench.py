@@ -357,7 +357,7 @@ def measure_convergent(V, n, steps, stream, dev, tol=1e-8):
         ms = e0.elapsed_time(e1)
         cells = prm.nx * prm.ny * prm.nz
         out[name] = {"value": round(cells * steps / (ms / 1e3) / 1e6, 1), "unit": UNIT,
-                     "ms_per_step": round(ms / steps, 4), "vcycles_per_step": round(float(np.mean(outer)), 2),
+                     "ms_per_step": round(ms / steps, 4), "corrections_per_step": round(float(np.mean(outer)), 2),
                      "max_rel_residual": float(np.max(rel)), "steps": steps,
                      "inner": "FP64 direct solve"}  # (from 8192 cells up, in both modes)
         fields[name] = s.state()

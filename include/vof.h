@@ -46,7 +46,8 @@ extern "C" {
 /* ---- solver modes ------------------------------------------------------ */
 #define VOF_MODE_PLAIN  0   /* FP32, jacobi_iters Jacobi sweeps: the drop-in path */
 /* Both: FP64 defect correction.  Grids of at least 8192 cells: each correction
-   is a direct FP64 solve (cosine transforms).  Smaller grids: one V-cycle, */
+   is a direct FP64 solve (cosine transforms).  Smaller grids, and boxes with planes
+   thousands of times closer than the cells of a row: one V-cycle, */
 #define VOF_MODE_MIXED  1   /* ... BF16-stored / FP32 arithmetic */
 #define VOF_MODE_FP64   2   /* ... FP64 */
 
